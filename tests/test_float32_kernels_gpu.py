@@ -1,4 +1,5 @@
-"""The 32-bit path's product at the edges of its tiles and of the rules that pick a kernel, against 64 bits."""
+"""The 32-bit path's product and attention at the edges of their tiles and of the rules that pick a kernel, against 64 bits."""
+import numpy as np
 import pytest
 import torch
 
@@ -47,3 +48,72 @@ def test_product_of_strided_and_misaligned_rows(ops, m):
     want = torch.empty(m, 133, device="cuda")
     ops.gemm_f32(a.contiguous(), w.contiguous(), want)
     assert torch.equal(out[:, 5:138], want) and not out[:, :5].any() and not out[:, 138:].any()
+
+
+def _attention_case(seed, lens, news, nh, nkv, d, page, planes, dtype):
+    """Requests that hold ``lens`` tokens of which the last ``news`` ask; pages in a shuffled order."""
+    from vllm_cpp_b200.cache.manager import cdiv
+    rng = np.random.default_rng(seed)
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    width = max(cdiv(n, page) for n in lens)
+    pages = sum(cdiv(n, page) for n in lens) + 1
+    order = rng.permutation(pages).tolist()
+    bt = np.full((len(lens), width), -1, dtype=np.int32)
+    rows = {}
+    cache = torch.zeros(pages, planes, nkv, page * d, dtype=dtype, device="cuda")
+    esize = 2 if dtype == torch.bfloat16 else 4
+
+    def place(slot):
+        e = np.arange(d)
+        if (d * esize) % 128:
+            return slot * d + e
+        per_plane, per_chunk = 128 // esize, 16 // esize
+        plane, w = e // per_plane, e % per_plane
+        return plane * page * per_plane + slot * per_plane + ((w // per_chunk) ^ (slot & 7)) * per_chunk + w % per_chunk
+
+    for r, n in enumerate(lens):
+        rows[r] = _rand(gen, n, planes, nkv, d).to(dtype)
+        for b in range(cdiv(n, page)):
+            bt[r, b] = order.pop()
+        for j in range(n):
+            cache[int(bt[r, j // page])][:, :, torch.from_numpy(place(j % page)).cuda()] = rows[r][j]
+    pos = np.concatenate([np.arange(n - k, n) for n, k in zip(lens, news)]).astype(np.int32)
+    req = np.concatenate([np.full(k, r) for r, k in enumerate(news)]).astype(np.int32)
+    q = _rand(gen, len(pos), nh, d).to(dtype)
+    return q, cache, rows, pos, req, bt
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,d,page,planes,window,sink", [
+    (2, 2, 4, 16, 2, 0, False), (6, 3, 16, 16, 2, 0, False), (7, 1, 32, 16, 2, 5, False), (18, 2, 36, 32, 2, 0, True), (16, 2, 64, 16, 1, 0, True),
+    (3, 3, 80, 48, 2, 70, False), (28, 4, 128, 16, 2, 0, False), (9, 1, 132, 16, 2, 0, True), (10, 2, 256, 16, 1, 33, False)])
+def test_attention_rows(ops, dtype, nh, nkv, d, page, planes, window, sink):
+    """Groups of one, two and more heads than a warp takes, rows of part of a warp's lanes and of two pieces a lane, keys shared among
+    several warps (few tokens) and not (many), windows, sinks, one plane."""
+    for lens, news in (([1, 130, 37], [1, 1, 1]), ([150, 61], [150, 40]), ([700], [700])):
+        if lens == [700] and (d > 64 or dtype == torch.bfloat16):
+            continue
+        q, cache, rows, pos, req, bt = _attention_case(nh + d, lens, news, nh, nkv, d, page, planes, dtype)
+        s = torch.randn(nh, device="cuda") if sink else None
+        out = torch.empty(len(pos), nh * d, dtype=dtype, device="cuda")
+        dev = lambda x: torch.from_numpy(x).cuda()  # noqa: E731
+        ops.attention_simt(q.view(len(pos), -1), cache, out, dev(pos), dev(req), dev(bt), num_heads=nh, num_kv_heads=nkv, head_dim=d,
+                           page_size=page, window=window, scale=d ** -0.5, planes=planes, sink=s)
+        want = torch.empty(len(pos), nh, d, dtype=torch.float64, device="cuda")
+        size = torch.empty(len(pos), nh, 1, dtype=torch.float64, device="cuda")
+        for r in range(len(lens)):
+            at = torch.from_numpy(np.nonzero(req == r)[0]).cuda()
+            p, j = torch.from_numpy(pos[req == r]).cuda()[:, None], torch.arange(lens[r], device="cuda")[None, :]
+            seen = (j <= p) & ((j > p - window) if window else (j >= 0))
+            for h in range(nh):
+                k, v = rows[r][:, 0, h // (nh // nkv)].double(), rows[r][:, -1, h // (nh // nkv)].double()
+                x = (q[at, h].double() @ k.T * d ** -0.5).masked_fill(~seen, -np.inf)
+                if sink:
+                    x = torch.cat([x, s[h].double().expand(len(at), 1)], 1)
+                w = torch.softmax(x, -1)[:, : lens[r]]
+                want[at, h] = w @ v
+                size[at, h] = w @ v.abs().amax(-1, keepdim=True)
+        # float: scores of size 10 carry about 10 * 2^-22 into the weights; the stored result is rounded once more in bfloat16
+        tol = 2e-5 if dtype == torch.float32 else 2e-5 + 2.0 ** -8
+        assert bool(((out.view(len(pos), nh, d).double() - want).abs() <= tol * size.clamp(min=1.0)).all())
+    ops.check_status()
