@@ -346,10 +346,11 @@ struct Engine::Impl {
             kernel_check(vcb_repetition_penalty(lg, mc.vocab, pen_ids_dev, pen_start_dev, samp_dev + 3 * cap, m, mc.vocab, stream),
                          "repetition_penalty");
         }
-        kernel_check(vcb_sample(lg, mc.vocab, mc.vocab, samp_dev, samp_dev + cap, ids_dev, m, stream), "sample");
         if (any_filter)
-            kernel_check(vcb_sample_filtered(lg, mc.vocab, mc.vocab, samp_dev, samp_dev + cap, samp_dev + 2 * cap, topk_dev, filter_scratch,
-                                             ids_dev, m, stream), "sample_filtered");
+            kernel_check(vcb_sample_all(lg, mc.vocab, mc.vocab, samp_dev, samp_dev + cap, samp_dev + 2 * cap, topk_dev, filter_scratch,
+                                        ids_dev, m, stream), "sample_all");
+        else
+            kernel_check(vcb_sample(lg, mc.vocab, mc.vocab, samp_dev, samp_dev + cap, ids_dev, m, stream), "sample");
         cuda_check(cudaMemcpyAsync(ids_host, ids_dev, m * 4, cudaMemcpyDeviceToHost, stream), "copy of the sampled ids");
         cuda_check(cudaStreamSynchronize(stream), "waiting for the step");
         if (++steps_since_check >= 64) {

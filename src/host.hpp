@@ -66,7 +66,7 @@ int vcb_repetition_penalty(float* logits, int ld, const int* ids, const int* row
                            int vocab, void* stream);
 int vcb_sample(const float* logits, int ld, int vocab, const float* temperature, const float* uniform, int* out, int n_rows,
                void* stream);
-int vcb_sample_filtered(const float* logits, int ld, int vocab, const float* temperature, const float* uniform,
+int vcb_sample_all(const float* logits, int ld, int vocab, const float* temperature, const float* uniform,
                         const float* top_p, const int* top_k, float* scratch, int* out, int n_rows, void* stream);
 }
 

@@ -49,6 +49,7 @@ _SIGNATURES = {
     "vcb_repetition_penalty": [_P, _I, _P, _P, _P, _I, _I, _P],
     "vcb_sample": [_P, _I, _I, _P, _P, _P, _I, _P],
     "vcb_sample_filtered": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P],
+    "vcb_sample_all": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P],
     "vcb_random_normal": [_P, ctypes.c_ulonglong, ctypes.c_ulonglong, ctypes.c_ulonglong, _F, _F, _I, _P],
     "vcb_attention_simt_planes": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P, _I, _I, _P],
     "vcb_attention_decode_mma_planes": [_P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _I, _I, _P],
@@ -1924,9 +1925,7 @@ def sample(logits, temperature, uniform, out) -> None:
 _filter_scratch: Optional[torch.Tensor] = None
 
 
-def sample_filtered(logits, temperature, uniform, top_p, top_k, out, scratch: Optional[torch.Tensor] = None) -> None:
-    """Redraws, in place in ``out``, the rows that have top-k or top-p set (see sampling.cu).
-    ``scratch``: float32, at least rows * vocab elements; one is kept and grown here if not given."""
+def _sample_rows(entry: str, logits, temperature, uniform, top_p, top_k, out, scratch) -> None:
     global _filter_scratch
     n, vocab = logits.shape
     _need(logits.is_cuda and logits.dtype == torch.float32 and logits.stride(1) == 1, "logits must be float32 rows")
@@ -1935,12 +1934,23 @@ def sample_filtered(logits, temperature, uniform, top_p, top_k, out, scratch: Op
         if _filter_scratch is None or _filter_scratch.numel() < n * vocab or _filter_scratch.device != logits.device:
             _filter_scratch = torch.empty(n * vocab, dtype=torch.float32, device=logits.device)
         scratch = _filter_scratch
-    _need(scratch.numel() >= n * vocab, "sample_filtered: scratch too small")
-    _check(lib().vcb_sample_filtered(logits.data_ptr(), logits.stride(0), vocab,
-                                     _dev(temperature, "temperature", torch.float32),
-                                     _dev(uniform, "uniform", torch.float32), _dev(top_p, "top_p", torch.float32),
-                                     _dev(top_k, "top_k", torch.int32), _dev(scratch, "scratch", torch.float32),
-                                     _dev(out, "out", torch.int32), n, _stream()), "sample_filtered")
+    _need(scratch.numel() >= n * vocab, f"{entry[4:]}: scratch too small")
+    _check(getattr(lib(), entry)(logits.data_ptr(), logits.stride(0), vocab,
+                                 _dev(temperature, "temperature", torch.float32),
+                                 _dev(uniform, "uniform", torch.float32), _dev(top_p, "top_p", torch.float32),
+                                 _dev(top_k, "top_k", torch.int32), _dev(scratch, "scratch", torch.float32),
+                                 _dev(out, "out", torch.int32), n, _stream()), entry[4:])
+
+
+def sample_filtered(logits, temperature, uniform, top_p, top_k, out, scratch: Optional[torch.Tensor] = None) -> None:
+    """Redraws, in place in ``out``, the rows that have top-k or top-p set (see sampling.cu).
+    ``scratch``: float32, at least rows * vocab elements; one is kept and grown here if not given."""
+    _sample_rows("vcb_sample_filtered", logits, temperature, uniform, top_p, top_k, out, scratch)
+
+
+def sample_all(logits, temperature, uniform, top_p, top_k, out, scratch: Optional[torch.Tensor] = None) -> None:
+    """``sample`` and then ``sample_filtered``, in one launch."""
+    _sample_rows("vcb_sample_all", logits, temperature, uniform, top_p, top_k, out, scratch)
 
 
 _scratch = {}

@@ -121,10 +121,11 @@ class Sampler:
             ops.repetition_penalty(logits, d_ids, d_start, d_float[3, :m].contiguous())
 
         out = self.d_out[slot][:m]
-        ops.sample(logits, temperature.contiguous(), uniform.contiguous(), out)
         if filtered:
-            ops.sample_filtered(logits, temperature.contiguous(), uniform.contiguous(),
-                                d_float[2, :m].contiguous(), d_int[0, :m].contiguous(), out)
+            ops.sample_all(logits, temperature.contiguous(), uniform.contiguous(),
+                           d_float[2, :m].contiguous(), d_int[0, :m].contiguous(), out)
+        else:
+            ops.sample(logits, temperature.contiguous(), uniform.contiguous(), out)
         self.h_out[slot][:m].copy_(out, non_blocking=True)
         self.events[slot].record()
         return SampleHandle(slot, m, self.events[slot])
