@@ -6,7 +6,8 @@
 //                            their sum and scaled (RouteRule)
 //   moe_sort_kernel          the (token, choice) pairs grouped by expert: a row for each pair in a list sorted by
 //                            expert, and the list's tiles of up to TM rows of one expert
-//   moe_expert_gemm_kernel   one product per tile against that expert's matrix; the first product gathers the
+//   moe_expert_gemm_kernel   (FMA; moe_expert_mma_kernel: mma.sync; moe_expert_tc_kernel: tcgen05, tiles of 128 rows)
+//                            one product per tile against that expert's matrix; the first product gathers the
 //                            tokens' rows, computes gate and up together and applies the experts' activation
 //                              g = min(gate, limit), u = clamp(up, -limit, limit), y = g * sigmoid(alpha * g) * (u + up_shift)
 //                            (limit = inf, alpha = 1, up_shift = 0: silu(gate) * up); or, for experts without a gate, one
@@ -19,6 +20,8 @@
 // same launches serve every routing (and a captured step).  Router, softmax, weights and all sums are float.
 // The reference has no routed feed-forward (src/layers/mlp.cpp is dense).
 #include "common.cuh"
+
+#include <cuda.h>
 
 // ------------------------------------------------------------------------------------------- router
 // Two kernels.  Logits: a CTA takes RT_TOK tokens and eight router outputs, a warp per output: the tokens' rows pass
@@ -498,6 +501,279 @@ moe_expert_mma_kernel(const __nv_bfloat16* __restrict__ A, long long lda, const 
                     ((float*)Cv)[(size_t)(r0 + m) * ldc + n] = acc[mi][nf][c];
                 }
             }
+}
+
+// The same products for steps with many rows per expert, on tcgen05: a CTA owns 128 rows of a tile and 256 columns (gated: 128
+// gate columns and the 128 up columns of the same features), whose sums stand in tensor memory (256 of its 512 columns: two CTAs share an
+// SM, so that one's epilogue and start run under the other's products).  Per 64-deep k slice 16 KB of rows and 32 KB of the
+// expert's matrix pass through shared memory in the 128-byte swizzle that the tensor cores read: the matrix by TMA (warp 0),
+// the rows, which lie anywhere, by 16-byte asynchronous copies of warps 2 to 5, eight lanes a row; warp 1 issues the
+// products.  Afterwards warps 2 to 5 read the sums back, a thread a row, apply the activation and store.
+// What bounds it is what an SM takes in from L2: 48 KB per 4.2 MFLOP.  2,048 tokens on 4 of 32 experts of 2,048, width 4,096: gate and
+// up 323 us (824 TFLOP/s), down 186 us (mma.sync tiles of 64 rows, whose 64 x 128 columns load 24 KB per 1.0 MFLOP: 1,189 and 681 us).
+// Every wait on an mbarrier is bounded; one that runs out is recorded in the status word and the CTA leaves without storing.
+namespace tc {
+
+constexpr int TM = 128, BN = 256, BK = 64, STAGES = 2, THREADS = 192;
+constexpr int A_BYTES = TM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + TM * 4;
+enum { STATUS_TIMEOUT = 14 };
+
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+// Shared-memory matrix descriptor of K-major rows of 128 bytes in the 128-byte swizzle, 8-row groups 1024 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFF) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// (the caller waits with wait_ld before it uses v)
+__device__ __forceinline__ void ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+template <int MODE>
+__global__ void __launch_bounds__(THREADS)
+moe_expert_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __nv_bfloat16* __restrict__ A, long long lda, void* __restrict__ Cv,
+                     long long ldc, int N, int K, const int* __restrict__ sorted_token, const int* __restrict__ tile_expert,
+                     const int* __restrict__ tile_row0, const int* __restrict__ tile_rows, const int* __restrict__ meta,
+                     float limit, float alpha, float up_shift, const float* __restrict__ row_scale, int* status) {
+    constexpr bool GATED = MODE == MG_GATED, GATHER = MODE != MG_PLAIN;
+    constexpr int COLS = GATED ? BN / 2 : BN;              // columns of C that the CTA stores
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+    const uint32_t full0 = cx_smem(bars), empty0 = cx_smem(bars + STAGES), done = cx_smem(bars + 2 * STAGES);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
+    volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const uint32_t stage0 = cx_smem(smem);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_wait();
+    const int tile = blockIdx.y;
+    if (tile >= meta[0]) return;
+    const int e = tile_expert[tile], r0 = tile_row0[tile], rows = tile_rows[tile], n0 = blockIdx.x * COLS;
+    const int steps = (K + BK - 1) / BK;
+
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; ++s) { cx_mbar_init(full0 + 8 * s, 1 + 128); cx_mbar_init(empty0 + 8 * s, 1); }
+        cx_mbar_init(done, 1);
+        *failed = 0;
+        cx_mbar_init_fence();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(cx_smem(tmem_slot)), "r"(BN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem_d = *tmem_slot;
+    // Not before: a following kernel that takes its tensor memory first and then waits for this grid would leave none for this CTA.
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const int b0 = e * (GATED ? 2 : 1) * N + n0, b1 = GATED ? b0 + N : b0 + BN / 2;
+            for (int it = 0; it < steps; ++it) {
+                const int s = it % STAGES;
+                if (*failed || !cx_mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1)) { *failed = 1; break; }
+                const uint32_t dst = stage0 + s * STAGE_BYTES + A_BYTES;
+                cx_mbar_expect_tx(full0 + 8 * s, B_BYTES);
+                tma_load(dst, &map_w, full0 + 8 * s, it * BK, b0);
+                tma_load(dst + B_BYTES / 2, &map_w, full0 + 8 * s, it * BK, b1);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // float accumulator, bfloat16 operands, both K-major, N and M
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+            for (int it = 0; it < steps; ++it) {
+                const int s = it % STAGES;
+                if (*failed || !cx_mbar_wait(full0 + 8 * s, (it / STAGES) & 1)) { *failed = 1; break; }
+                fence_after();
+                const uint32_t pa = stage0 + s * STAGE_BYTES, pb = pa + A_BYTES;
+#pragma unroll
+                for (int j = 0; j < BK / 16; ++j) mma(tmem_d, smem_desc(pa + j * 32), smem_desc(pb + j * 32), idesc, (it > 0 || j > 0) ? 1u : 0u);
+                commit(empty0 + 8 * s);
+            }
+            commit(done);
+        }
+    } else {
+        // ---- rows: eight threads a row, 16 rows a round
+        const int t = tid - 64, c = t & 7, row0 = t >> 3;
+        const __nv_bfloat16* src[TM / 16];
+#pragma unroll
+        for (int i = 0; i < TM / 16; ++i) {
+            const int r = row0 + 16 * i;
+            src[i] = r < rows ? A + (size_t)(GATHER ? sorted_token[r0 + r] : r0 + r) * lda + c * 8 : nullptr;
+        }
+        const uint32_t at = row0 * 128 + ((c ^ (row0 & 7)) << 4);          // (row0 + 16 i) % 8 is row0 % 8
+        bool ok = true;
+        for (int it = 0; it < steps + STAGES - 1; ++it) {
+            if (it < steps) {
+                const int s = it % STAGES;
+                ok = ok && !*failed && cx_mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1);
+                if (!ok) { *failed = 1; break; }
+                const uint32_t dst = stage0 + s * STAGE_BYTES + at;
+                const int k = it * BK + c * 8;
+#pragma unroll
+                for (int i = 0; i < TM / 16; ++i) {
+                    const bool valid = src[i] != nullptr && k < K;
+                    const int bytes = valid ? 16 : 0;
+                    const void* from = valid ? (const void*)(src[i] + it * BK) : (const void*)A;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * 2048), "l"(from), "r"(bytes) : "memory");
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (it >= STAGES - 1) {                        // the copies of step it - (STAGES - 1) are there: show them to the tensor cores
+                asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                cx_mbar_arrive(full0 + 8 * ((it - (STAGES - 1)) % STAGES));
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // ---- epilogue: warps 2..5 own tensor-memory lanes 32 * (warp % 4) ..
+        if (ok && cx_mbar_wait(done, 0) && !*failed) {
+            fence_after();
+            const int row = (warp & 3) * 32 + lane;
+            const bool store = row < rows;
+            const uint32_t base = tmem_d + ((uint32_t)((warp & 3) * 32) << 16);
+            const float scale = MODE == MG_GELU && row_scale && store ? row_scale[r0 + row] : 1.0f;
+            const bool whole = n0 + COLS <= N && (ldc % 8) == 0 && (((uintptr_t)Cv) & 15) == 0;
+#pragma unroll 1
+            for (int n = 0; n < COLS; n += 16) {
+                uint32_t g[16], u[16];
+                __syncwarp();
+                ld16(base + n, g);
+                if (GATED) ld16(base + BN / 2 + n, u);
+                wait_ld();
+                if (!store) continue;
+                float y[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float x = __uint_as_float(g[j]);
+                    if (GATED) {
+                        const float gg = fminf(x, limit), uu = fminf(fmaxf(__uint_as_float(u[j]), -limit), limit);
+                        y[j] = gg * (1.0f / (1.0f + expf(-alpha * gg))) * (uu + up_shift);
+                    } else if (MODE == MG_GELU) {
+                        y[j] = gelu_erf(x * scale);
+                    } else {
+                        y[j] = x;
+                    }
+                }
+                const size_t off = (size_t)(r0 + row) * ldc + n0 + n;
+                if (MODE == MG_PLAIN) {
+                    float* o = (float*)Cv + off;
+                    if (whole) {
+#pragma unroll
+                        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
+                    } else {
+                        for (int j = 0; j < 16; ++j)
+                            if (n0 + n + j < N) o[j] = y[j];
+                    }
+                } else {
+                    __nv_bfloat16* o = (__nv_bfloat16*)Cv + off;
+                    if (whole) {
+                        uint32_t w[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const __nv_bfloat162 v = __floats2bfloat162_rn(y[2 * j], y[2 * j + 1]);
+                            w[j] = *reinterpret_cast<const uint32_t*>(&v);
+                        }
+                        *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+                        *reinterpret_cast<uint4*>(o + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                    } else {
+                        for (int j = 0; j < 16; ++j)
+                            if (n0 + n + j < N) o[j] = __float2bfloat16_rn(y[j]);
+                    }
+                }
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (*failed) {
+        // loads that were requested must land before the CTA's shared memory goes: a stage whose phase never completes is given up
+        if (tid == 0) {
+            if (status) atomicCAS(status, 0, STATUS_TIMEOUT);
+            for (int s = 0; s < STAGES; ++s) cx_mbar_wait(full0 + 8 * s, 0);
+            cx_mbar_wait(done, 0);                         // products still under way read shared and write tensor memory
+        }
+        __syncthreads();
+    }
+    if (warp == 1) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(BN) : "memory");
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// The experts' matrices as one [rows, K] matrix read in boxes of 64 x 128 with 128-byte swizzle.
+static int make_map(CUtensorMap* map, const void* base, long long rows, int K) {
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            return VCB_ERR_UNSUPPORTED;
+        fn = reinterpret_cast<EncodeTiledFn>(p);
+    }
+    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+    cuuint32_t box[2] = {BK, BN / 2}, estr[2] = {1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : VCB_ERR_BAD_ARG;
+}
+
+template <int MODE, typename... Args>
+static int launch(const CUtensorMap& map, dim3 grid, cudaStream_t s, Args... args) {
+    static unsigned long long done = 0;
+    if (int e = vcb_allow_dynamic_smem(moe_expert_tc_kernel<MODE>, SMEM, &done)) return e;
+    vcb_launch(moe_expert_tc_kernel<MODE>, grid, THREADS, SMEM, s, map, args...);
+    return vcb_last_error();
+}
+
+}  // namespace tc
+
+// The experts' products over tiles of 128 rows (moe_sort's tm) in bfloat16; n_experts: how many matrices W holds.
+// K a multiple of 8, rows of A and W at 16-byte boundaries.  status: the device word for waits that ran out.  The rest as below.
+VCB_EXPORT int vcb_moe_expert_gemm_tc(const void* A, long long lda, const void* W, int n_experts, void* C, long long ldc, int N, int K,
+                                      const int* sorted_token, const int* tile_expert, const int* tile_row0, const int* tile_rows,
+                                      const int* meta, int max_tiles, int mode, float limit, float alpha, float up_shift,
+                                      const float* row_scale, int* status, void* stream) {
+    if (max_tiles <= 0) return 0;
+    if (!A || !W || !C || N <= 0 || K <= 0 || n_experts <= 0 || max_tiles > 65535 || mode < MG_PLAIN || mode > MG_GELU) return VCB_ERR_BAD_ARG;
+    if (K % 8 || lda % 8 || (((uintptr_t)A | (uintptr_t)W) & 15)) return VCB_ERR_UNSUPPORTED;
+    const long long rows = (long long)n_experts * N * (mode == MG_GATED ? 2 : 1);
+    if (rows + tc::BN > 0x7fffffffLL) return VCB_ERR_UNSUPPORTED;
+    CUtensorMap map;
+    if (int e = tc::make_map(&map, W, rows, K)) return e;
+    const int cols = mode == MG_GATED ? tc::BN / 2 : tc::BN;
+    dim3 grid((N + cols - 1) / cols, max_tiles);
+    cudaStream_t s = (cudaStream_t)stream;
+#define MOE_TC(M) tc::launch<M>(map, grid, s, (const __nv_bfloat16*)A, lda, C, ldc, N, K, sorted_token, tile_expert, tile_row0, tile_rows, meta, \
+                                limit, alpha, up_shift, row_scale, status)
+    return mode == MG_GATED ? MOE_TC(MG_GATED) : mode == MG_GELU ? MOE_TC(MG_GELU) : MOE_TC(MG_PLAIN);
+#undef MOE_TC
 }
 
 // mode MG_GATED (1): A = the tokens' rows [n, K] (T), W [E, 2 * N, K], C [pairs, N] (T).  MG_GELU (2): A the tokens' rows, W [E,
