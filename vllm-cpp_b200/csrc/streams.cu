@@ -65,6 +65,103 @@ __global__ void stream_norm_kernel(StreamNormArgs a) {
     }
 }
 
+// Both for SN streams and rows of whole 16-byte pieces: a thread holds its pieces of the combined row in registers (PER of them, up to eight of 4 floats
+// each), loads are 16 bytes wide and all streams' loads of a piece are in flight at once, so the row is read once and never goes
+// through shared memory.  Bound by memory for many rows (2,048 rows of 4 x 4,096: 53 us, 99 us with 4-byte accesses through shared memory),
+// by two block-wide sums for few (8 rows: 4.6 us, 9.4).
+template <typename T> __device__ __forceinline__ float4 load4(const T* p);
+template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
+template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+__device__ __forceinline__ float4 fma4(float c, float4 x, float4 y) {
+    return make_float4(fmaf(c, x.x, y.x), fmaf(c, x.y, y.y), fmaf(c, x.z, y.z), fmaf(c, x.w, y.w));
+}
+
+// u[k]: the thread's pieces (zero beyond the row).  Two passes, as row_statistics.
+template <int PER>
+__device__ __forceinline__ void piece_statistics(const float4 (&u)[PER], int pieces, int hidden, float eps, float* scratch, float& mean, float& rstd) {
+    float s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) s += (u[k].x + u[k].y) + (u[k].z + u[k].w);
+    mean = block_sum(s, scratch) / (float)hidden;
+    float v = 0.0f;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        if ((int)threadIdx.x + k * (int)blockDim.x >= pieces) break;
+        const float a = u[k].x - mean, b = u[k].y - mean, c = u[k].z - mean, d = u[k].w - mean;
+        v += (a * a + b * b) + (c * c + d * d);
+    }
+    rstd = 1.0f / sqrtf(block_sum(v, scratch) / (float)hidden + eps);
+}
+
+template <typename T, int PER>
+__device__ __forceinline__ void store_normed(const float4 (&u)[PER], int pieces, float mean, float rstd, const float* w, const float* b, float scale, T* dst) {
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i >= pieces) break;
+        const float4 g = load4<float>(w + 4 * i), c = b ? load4<float>(b + 4 * i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        store4<T>(dst + 4 * i, make_float4(((u[k].x - mean) * rstd * g.x + c.x) * scale, ((u[k].y - mean) * rstd * g.y + c.y) * scale,
+                                           ((u[k].z - mean) * rstd * g.z + c.z) * scale, ((u[k].w - mean) * rstd * g.w + c.w) * scale));
+    }
+}
+
+template <typename T, int SN, int PER>
+__global__ void __launch_bounds__(512)
+stream_norm_vec_kernel(StreamNormArgs a) {
+    __shared__ float scratch[33];
+    pdl_start();
+    const int o = blockIdx.x, row = a.row_index ? a.row_index[o] : o, pieces = a.hidden / 4;
+    float c[SN];
+#pragma unroll
+    for (int s = 0; s < SN; ++s) c[s] = a.coef[s];
+    const float* x = a.x + (size_t)row * a.hidden;
+    float4 u[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        u[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i >= pieces) continue;
+        float4 v[SN];
+#pragma unroll
+        for (int s = 0; s < SN; ++s) v[s] = load4<float>(x + (size_t)s * a.stream_stride + 4 * i);
+#pragma unroll
+        for (int s = 0; s < SN; ++s) u[k] = fma4(c[s], v[s], u[k]);
+    }
+    float mean, rstd;
+    piece_statistics<PER>(u, pieces, a.hidden, a.eps, scratch, mean, rstd);
+    store_normed<T, PER>(u, pieces, mean, rstd, a.w, a.b, a.out_scale, (T*)a.out + (size_t)o * a.hidden);
+}
+
+// Threads of a row's CTA, and 16-byte pieces of it a thread holds.  512 threads of two pieces at 4,096 elements: 1,024 of one have fewer
+// loads in flight each and leave an SM room for one row less (2,048 rows 77 against 53 us), 256 of four wait longer for few rows (8
+// rows 5.8 against 4.6).
+static inline bool stream_pieces(int hidden, int& threads, int& per) {
+    if (hidden % 4 || hidden > 16384) return false;
+    const int pieces = hidden / 4;
+    threads = pieces >= 512 ? 512 : (pieces + 31) / 32 * 32;
+    per = (pieces + threads - 1) / threads;
+    per = per > 4 ? 8 : per > 2 ? 4 : per;
+    return true;
+}
+static inline bool aligned16(const void* a, const void* b, const void* c, const void* d, const void* e) {
+    return ((((uintptr_t)a) | ((uintptr_t)b) | ((uintptr_t)c) | ((uintptr_t)d) | ((uintptr_t)e)) & 15) == 0;
+}
+#define STREAM_CASES(GO, T) do { \
+        if (S == 4) { if (per == 1) GO(T, 4, 1); else if (per == 2) GO(T, 4, 2); else if (per == 4) GO(T, 4, 4); else GO(T, 4, 8); } \
+        else if (S == 2) { if (per == 1) GO(T, 2, 1); else if (per == 2) GO(T, 2, 2); else if (per == 4) GO(T, 2, 4); else GO(T, 2, 8); } \
+        else { if (per == 1) GO(T, 1, 1); else if (per == 2) GO(T, 1, 2); else if (per == 4) GO(T, 1, 4); else GO(T, 1, 8); } \
+    } while (0)
+
 VCB_EXPORT int vcb_stream_norm(const float* x, long long stream_stride, const float* coef, const float* w, const float* b,
                                void* out, const int* row_index, int rows, int S, int hidden, float eps, float out_scale,
                                int dtype, void* stream) {
@@ -73,6 +170,15 @@ VCB_EXPORT int vcb_stream_norm(const float* x, long long stream_stride, const fl
     const size_t smem = (size_t)hidden * sizeof(float);
     if (smem > 200 * 1024) return VCB_ERR_UNSUPPORTED;
     StreamNormArgs a{x, stream_stride, coef, w, b, out, row_index, S, hidden, eps, out_scale};
+    int wide, per;
+    if ((S == 1 || S == 2 || S == 4) && (dtype == VCB_F32 || dtype == VCB_BF16) && stream_stride % 4 == 0 && aligned16(x, w, b, out, nullptr) &&
+        stream_pieces(hidden, wide, per)) {
+#define STREAM_NORM(T, SN, PN) vcb_launch(stream_norm_vec_kernel<T, SN, PN>, rows, wide, 0, (cudaStream_t)stream, a)
+        if (dtype == VCB_F32) STREAM_CASES(STREAM_NORM, float);
+        else STREAM_CASES(STREAM_NORM, __nv_bfloat16);
+#undef STREAM_NORM
+        return vcb_last_error();
+    }
     const int threads = hidden >= 4096 ? 512 : hidden >= 1024 ? 256 : 128;
     cudaStream_t s = (cudaStream_t)stream;
     static unsigned long long done_f = 0, done_b = 0;
@@ -147,6 +253,49 @@ __global__ void stream_join_kernel(StreamJoinArgs a) {
         dst[i] = from_f32<T>((u[i] - mean) * rstd * a.next_w[i] + (a.next_b ? a.next_b[i] : 0.0f));
 }
 
+template <typename T, int SN, int PER>
+__global__ void __launch_bounds__(512)
+stream_join_vec_kernel(StreamJoinArgs a) {
+    __shared__ float scratch[33];
+    // the coefficients are weights: read ahead of the kernel before
+    float mix[SN][SN], oc[SN], nc[SN];
+#pragma unroll
+    for (int s = 0; s < SN; ++s) {
+        oc[s] = a.out_coef[s];
+        nc[s] = a.next_out ? a.next_coef[s] : 0.0f;
+#pragma unroll
+        for (int t = 0; t < SN; ++t) mix[s][t] = a.mix[s * SN + t];
+    }
+    pdl_start();
+    const size_t row = (size_t)blockIdx.x * a.hidden;
+    const int pieces = a.hidden / 4;
+    float* x = a.x + row;
+    const T* y = (const T*)a.y + row;
+    float4 u[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        u[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i >= pieces) continue;
+        float4 old[SN];
+#pragma unroll
+        for (int s = 0; s < SN; ++s) old[s] = load4<float>(x + (size_t)s * a.stream_stride + 4 * i);
+        const float4 yv = load4<T>(y + 4 * i);
+#pragma unroll
+        for (int t = 0; t < SN; ++t) {
+            float4 v = make_float4(oc[t] * yv.x, oc[t] * yv.y, oc[t] * yv.z, oc[t] * yv.w);
+#pragma unroll
+            for (int s = 0; s < SN; ++s) v = fma4(mix[s][t], old[s], v);
+            store4<float>(x + (size_t)t * a.stream_stride + 4 * i, v);
+            u[k] = fma4(nc[t], v, u[k]);
+        }
+    }
+    if (!a.next_out) return;
+    float mean, rstd;
+    piece_statistics<PER>(u, pieces, a.hidden, a.eps, scratch, mean, rstd);
+    store_normed<T, PER>(u, pieces, mean, rstd, a.next_w, a.next_b, 1.0f, (T*)a.next_out + row);
+}
+
 VCB_EXPORT int vcb_stream_join(float* x, long long stream_stride, const void* y, const float* mix, const float* out_coef,
                                const float* next_coef, const float* next_w, const float* next_b, void* next_out, int n,
                                int S, int hidden, float eps, int dtype, void* stream) {
@@ -156,6 +305,15 @@ VCB_EXPORT int vcb_stream_join(float* x, long long stream_stride, const void* y,
     const size_t smem = next_out ? (size_t)hidden * sizeof(float) : 0;
     if (smem > 200 * 1024) return VCB_ERR_UNSUPPORTED;
     StreamJoinArgs a{x, stream_stride, y, mix, out_coef, next_coef, next_w, next_b, next_out, S, hidden, eps};
+    int wide, per;
+    if ((S == 1 || S == 2 || S == 4) && (dtype == VCB_F32 || dtype == VCB_BF16) && stream_stride % 4 == 0 && aligned16(x, y, next_w, next_b, next_out) &&
+        stream_pieces(hidden, wide, per)) {
+#define STREAM_JOIN(T, SN, PN) vcb_launch(stream_join_vec_kernel<T, SN, PN>, n, wide, 0, (cudaStream_t)stream, a)
+        if (dtype == VCB_F32) STREAM_CASES(STREAM_JOIN, float);
+        else STREAM_CASES(STREAM_JOIN, __nv_bfloat16);
+#undef STREAM_JOIN
+        return vcb_last_error();
+    }
     const int threads = hidden >= 4096 ? 512 : hidden >= 1024 ? 256 : 128;
     cudaStream_t s = (cudaStream_t)stream;
     static unsigned long long done_f = 0, done_b = 0;
