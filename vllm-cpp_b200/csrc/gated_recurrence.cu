@@ -14,6 +14,7 @@
 //
 // States, decays and their logarithms, softplus and exponentials, gates, unit norms and every sum are float whatever the
 // type T of the projections is.  The reference has no recurrent mixer (src/layers/attention.cpp is its only mixer).
+#include "fast_math.cuh"
 #include "short_conv.cuh"
 
 #define CONV_MAX_TAPS 64       // up to 8 in registers (short_conv.cuh), more from memory
@@ -224,6 +225,116 @@ gate_blocks_kernel(const float* __restrict__ u, long long ldu, const T* __restri
     }
 }
 
+// The same where blocks and rows are whole 16-byte pieces: 128 threads of 8 tokens x 4 channels x both matrices as packed pairs, operands
+// k-major in shared memory and read 16 bytes at a time, the next slice's loads in flight while this one is used.  Bound by the FMA pipe and
+// the shared-memory reads alike (four of 16 bytes per 32 packed FMAs).  2,048 tokens, 32 blocks of 128: 149 us, 235 us with 4 x 4 sums a
+// thread and 4-byte reads.
+template <typename T> __device__ __forceinline__ void gate_piece8(const T* p, float (&v)[8]);
+template <> __device__ __forceinline__ void gate_piece8<float>(const float* p, float (&v)[8]) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+template <> __device__ __forceinline__ void gate_piece8<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) {
+    const uint4 x = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128)
+gate_tiles_kernel(const float* __restrict__ u, long long ldu, const T* __restrict__ wa, const T* __restrict__ wi,
+                  const float* __restrict__ ba, const float* __restrict__ bi, const float* __restrict__ lam,
+                  float* __restrict__ decay, float* __restrict__ drive, long long ldo, int n, int bs, int tiles_per_block, float c_gate) {
+    constexpr int KS = 16, LD = 68;
+    __shared__ __align__(16) float Us[2][KS][LD];
+    __shared__ __align__(16) float As[2][KS][LD];
+    __shared__ __align__(16) float Is[2][KS][LD];
+    pdl_start();
+    const int b = blockIdx.y / tiles_per_block, n0 = (blockIdx.y % tiles_per_block) * 64, t0 = blockIdx.x * 64;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;                // channels 4 tx .., tokens 8 ty ..
+    const int row = threadIdx.x >> 1, half = (threadIdx.x & 1) * 8;        // a thread stages eight k's of a row of each operand
+    const T* Wa = wa + (size_t)b * bs * bs;
+    const T* Wi = wi + (size_t)b * bs * bs;
+    const float* ub = u + (size_t)b * bs;
+    float su[8], sa[8], si[8];
+    auto fetch = [&](int k0) {
+        const int k = k0 + half;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) su[e] = sa[e] = si[e] = 0.0f;
+        if (k >= bs) return;                                               // bs is a multiple of 8
+        if (t0 + row < n) gate_piece8<float>(ub + (size_t)(t0 + row) * ldu + k, su);
+        if (n0 + row < bs) {
+            gate_piece8<T>(Wa + (size_t)(n0 + row) * bs + k, sa);
+            gate_piece8<T>(Wi + (size_t)(n0 + row) * bs + k, si);
+        }
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { Us[buf][half + e][row] = su[e]; As[buf][half + e][row] = sa[e]; Is[buf][half + e][row] = si[e]; }
+    };
+    f32x2 accr[8][2], acci[8][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) accr[i][j] = acci[i][j] = 0ull;        // (0.0f, 0.0f)
+    fetch(0);
+    put(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < bs; k0 += KS, buf ^= 1) {
+        const bool more = k0 + KS < bs;
+        if (more) fetch(k0 + KS);
+#pragma unroll
+        for (int kk = 0; kk < KS; ++kk) {
+            const float4 x = *reinterpret_cast<const float4*>(&Us[buf][kk][ty * 8]), y = *reinterpret_cast<const float4*>(&Us[buf][kk][ty * 8 + 4]);
+            const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(&As[buf][kk][tx * 4]), iv = *reinterpret_cast<const ulonglong2*>(&Is[buf][kk][tx * 4]);
+            const float uv[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const f32x2 uu = pack2f(uv[i], uv[i]);
+                accr[i][0] = fma2f(uu, av.x, accr[i][0]);
+                accr[i][1] = fma2f(uu, av.y, accr[i][1]);
+                acci[i][0] = fma2f(uu, iv.x, acci[i][0]);
+                acci[i][1] = fma2f(uu, iv.y, acci[i][1]);
+            }
+        }
+        if (more) put(buf ^ 1);                                            // read last before the barrier that ended the slice before
+        __syncthreads();
+    }
+    const int cb = n0 + tx * 4, c = b * bs + cb;
+    if (cb >= bs) return;                                                  // four channels or none: bs is a multiple of 8
+    float sp[4], bav[4], biv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { sp[j] = gr_softplus(lam[c + j]); bav[j] = ba[c + j]; biv[j] = bi[c + j]; }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = t0 + ty * 8 + i;
+        if (t >= n) break;
+        float zr[4], zi[4], d[4], dr[4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            unpack2f(accr[i][j], zr[2 * j], zr[2 * j + 1]);
+            unpack2f(acci[i][j], zi[2 * j], zi[2 * j + 1]);
+        }
+        const float4 uv = *reinterpret_cast<const float4*>(u + (size_t)t * ldu + c);
+        const float uu[4] = {uv.x, uv.y, uv.z, uv.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float r = gr_sigmoid(zr[j] + bav[j]), g = gr_sigmoid(zi[j] + biv[j]);
+            const float la = -c_gate * r * sp[j];
+            d[j] = expf(la);
+            dr[j] = sqrtf(-expm1f(2.0f * la)) * g * uu[j];
+        }
+        *reinterpret_cast<float4*>(decay + (size_t)t * ldo + c) = make_float4(d[0], d[1], d[2], d[3]);
+        *reinterpret_cast<float4*>(drive + (size_t)t * ldo + c) = make_float4(dr[0], dr[1], dr[2], dr[3]);
+    }
+}
+
 // The same for a few tokens (single tokens of a batch) and blocks of up to GATE_ROWS_BS channels: the tiles above would
 // fill a fraction of the SMs and walk the block's inputs in dependent slices.  A warp per output channel: its lanes split
 // the block's inputs and keep their weights of both matrices in registers, every token costs two warp sums, and lane t % 32
@@ -310,6 +421,15 @@ VCB_EXPORT int vcb_gate_blocks(const float* u, long long ldu, const void* wa, co
         return vcb_last_error();
     }
     dim3 grid((n + 63) / 64, B * tiles);
+    const uintptr_t at = (uintptr_t)u | (uintptr_t)wa | (uintptr_t)wi | (uintptr_t)decay | (uintptr_t)drive;
+    if (bs % 8 == 0 && ldu % 4 == 0 && ldo % 4 == 0 && (at & 15) == 0 && (dtype == VCB_F32 || dtype == VCB_BF16)) {
+        if (dtype == VCB_F32)
+            vcb_launch(gate_tiles_kernel<float>, grid, 128, 0, s, u, ldu, (const float*)wa, (const float*)wi, ba, bi, lam, decay, drive, ldo, n, bs, tiles, c_gate);
+        else
+            vcb_launch(gate_tiles_kernel<__nv_bfloat16>, grid, 128, 0, s, u, ldu, (const __nv_bfloat16*)wa, (const __nv_bfloat16*)wi, ba, bi, lam,
+                       decay, drive, ldo, n, bs, tiles, c_gate);
+        return vcb_last_error();
+    }
     if (dtype == VCB_F32)
         vcb_launch(gate_blocks_kernel<float>, grid, 256, 0, s, u, ldu, (const float*)wa, (const float*)wi, ba, bi, lam, decay, drive, ldo, n, bs, tiles, c_gate);
     else if (dtype == VCB_BF16)
@@ -635,19 +755,199 @@ delta_prepare_kernel(DeltaArgs a, float* __restrict__ work, long long ldw, int n
     if (lane == 0) w[(2 * a.G + a.H) * dk + h] = gr_sigmoid(to_f32<T>(((const T*)a.beta_pre)[row * a.ldb + h]));
 }
 
-// delta_walk_kernel, grid (request, head, tile of DVT value channels), P lanes of a warp per column of S, DKP rows of
-// the column in a thread's registers.  With S' = diag(g) S, both sums over key channels that a token needs come from S':
+// delta_walk_kernel, grid (request, head, tile of DVT value channels), P lanes of a warp per COLS neighbouring columns of S, DKP rows
+// of each in a thread's registers as packed pairs.  With S' = diag(g) S, both sums over key channels that a token needs come from S':
 //   p = k . S'[:, c],  r = q . S'[:, c];   u = beta (v_c - p);   S[:, c] = S'[:, c] + k u;   o_c = r + (q . k) u
-// so a token costs one round of shuffles, for two sums at once.  Chunks of a.chunk tokens' rows go through shared memory.
+// so a token costs one round of sums over the lanes, and the eight sums of four columns are added up by halving: seven exchanges and one
+// more for 16 lanes, where a butterfly for each would take 32.  Chunks of a.chunk tokens' rows go through shared memory.
+// A row's q, k and g are read from shared memory once per four columns: with one column a thread those reads bound the walk
+// (32 heads of 128 x 128, eight prompts of together 2,048 tokens: 1,093 us, with four columns 645).
 __device__ __forceinline__ void walk_copy(float* smem, const float* gmem, int bytes) {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
     if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(gmem) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(gmem) : "memory");
 }
 
-template <int DKP>
+// s[0 .. N) summed over the lanes whose numbers differ in the bits from BIT down; lane l ends with sum l / (2 BIT / N) in s[0].
+template <int N>
+__device__ __forceinline__ void walk_halve(float* s, int part, int bit) {
+    if constexpr (N > 1) {
+        const bool upper = (part & bit) != 0;
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            const float keep = upper ? s[i + N / 2] : s[i], give = upper ? s[i] : s[i + N / 2];
+            s[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+        walk_halve<N / 2>(s, part, bit >> 1);
+    } else {
+        for (; bit >= 1; bit >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+    }
+}
+
+template <int DKP, int COLS>
 __global__ void __launch_bounds__(128)
 delta_walk_kernel(DeltaArgs a, const float* __restrict__ work, long long ldw, int P, int DVT) {
+    extern __shared__ __align__(16) float sm[];
+    pdl_start();
+    const int r = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * DVT;
+    const int kvh = h / (a.H / a.G);
+    const int tid = threadIdx.x, nthreads = blockDim.x;
+    const int part = tid % P, cl = tid / P * COLS;    // of 128 threads, P lanes a column group: DVT = 128 / P * COLS columns
+    const int col = col0 + cl;
+    const int pstride = DKP + 4, tstride = P * pstride, dk = a.dk, TC = a.chunk;
+    // two buffers of a chunk's rows, filled by asynchronous copies while the chunk before is walked:
+    // [q, k, g: TC x tstride each][v: TC x DVT][beta, q . k: TC x 2], then the chunk's outputs [TC x DVT]
+    const int buf_floats = TC * (3 * tstride + DVT + 2);
+    float* os = sm + 2 * buf_floats;
+    const int row0 = a.q_start[r], row1 = a.q_start[r + 1];
+    float* st = a.state + (((size_t)a.state_slots[r] * a.H + h) * dk) * a.dv;
+    f32x2 S[COLS][DKP / 2];
+#pragma unroll
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int i = 0; i < DKP / 2; ++i) {
+            const int kr = part * DKP + 2 * i;
+            const bool ok = col + c < a.dv;
+            S[c][i] = pack2f(ok && kr < dk ? st[(size_t)kr * a.dv + col + c] : 0.0f, ok && kr + 1 < dk ? st[(size_t)(kr + 1) * a.dv + col + c] : 0.0f);
+        }
+    const int off_q = kvh * dk, off_k = (a.G + kvh) * dk, off_g = (2 * a.G + h) * dk, off_b = (2 * a.G + a.H) * dk;
+    // key channels beyond dk: q = k = 0, g = 1, and value channels beyond dv: v = 0, written once (the copies never touch them)
+    for (int idx = tid; idx < 2 * TC * P * DKP; idx += nthreads) {
+        const int b = idx / (TC * P * DKP), rest = idx - b * (TC * P * DKP);
+        const int tt = rest / (P * DKP), i = rest - tt * (P * DKP);
+        if (i >= dk) {
+            float* base = sm + b * buf_floats + tt * tstride + (i / DKP) * pstride + i % DKP;
+            base[0] = 0.0f;
+            base[TC * tstride] = 0.0f;
+            base[2 * TC * tstride] = 1.0f;
+        }
+    }
+    for (int idx = tid; idx < 2 * TC * DVT; idx += nthreads) {
+        const int b = idx / (TC * DVT), rest = idx - b * (TC * DVT);
+        if (col0 + rest % DVT >= a.dv) sm[b * buf_floats + 3 * TC * tstride + rest] = 0.0f;
+    }
+    const bool wide = (dk & 3) == 0;               // rows of the prepared inputs start on 16 bytes, so do their heads then
+    const bool wide_v = (DVT & 3) == 0 && ((a.dv | (int)(a.ldv & 3)) & 3) == 0 && (((uintptr_t)a.v) & 15) == 0;
+    const int piece = wide ? 4 : 1, pieces = dk / piece, piece_v = wide_v ? 4 : 1, pieces_v = DVT / piece_v;
+    auto fetch = [&](int c0, int b) {
+        const int tc = min(TC, row1 - c0);
+        float* qs = sm + b * buf_floats;
+        float* vs = qs + 3 * TC * tstride;
+        float* bs = vs + TC * DVT;
+        for (int idx = tid; idx < tc * pieces; idx += nthreads) {
+            const int tt = idx / pieces, i = (idx - tt * pieces) * piece;
+            const float* w = work + (size_t)(c0 + tt) * ldw;
+            float* at = qs + tt * tstride + (i / DKP) * pstride + i % DKP;
+            walk_copy(at, w + off_q + i, 4 * piece);
+            walk_copy(at + TC * tstride, w + off_k + i, 4 * piece);
+            walk_copy(at + 2 * TC * tstride, w + off_g + i, 4 * piece);
+        }
+        for (int idx = tid; idx < tc * pieces_v; idx += nthreads) {
+            const int tt = idx / pieces_v, j = (idx - tt * pieces_v) * piece_v, c = col0 + j;
+            if (c < a.dv) walk_copy(vs + tt * DVT + j, a.v + (size_t)(c0 + tt) * a.ldv + h * a.dv + c, 4 * piece_v);
+        }
+        for (int idx = tid; idx < 2 * tc; idx += nthreads) {
+            const int tt = idx >> 1;
+            walk_copy(bs + idx, work + (size_t)(c0 + tt) * ldw + off_b + ((idx & 1) ? a.H + kvh : h), 4);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (row0 < row1) fetch(row0, 0);
+    const int rep = P / (2 * COLS);           // lanes that end with the same sum; P is at least 8
+    const int lane0 = (tid & 31) - part;           // the first lane of this column group
+    int b = 0;
+    for (int c0 = row0; c0 < row1; c0 += TC, b ^= 1) {
+        const int tc = min(TC, row1 - c0);
+        if (c0 + TC < row1) {
+            fetch(c0 + TC, b ^ 1);                 // its buffer was walked two chunks ago; the barriers since cover it
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();                           // everybody's copies of this chunk have landed; the outputs before are stored
+        const float* qs = sm + b * buf_floats;
+        const float* vs = qs + 3 * TC * tstride;
+        const float* bs = vs + TC * DVT;
+        // the rows of the token after this one are read from shared memory while this one's sums run; two sets of
+        // registers take turns, so nothing is copied between them
+        struct Rows { f32x2 q[DKP / 2], k[DKP / 2], g[DKP / 2]; float v[COLS], beta, qk; };
+        const float* mine = qs + part * pstride;
+        auto read = [&](Rows& w, int tt) {
+            const float* at = mine + tt * tstride;
+#pragma unroll
+            for (int i = 0; i < DKP / 4; ++i) {
+                const ulonglong2 q = reinterpret_cast<const ulonglong2*>(at)[i], k = reinterpret_cast<const ulonglong2*>(at + TC * tstride)[i],
+                                 g = reinterpret_cast<const ulonglong2*>(at + 2 * TC * tstride)[i];
+                w.q[2 * i] = q.x; w.q[2 * i + 1] = q.y;
+                w.k[2 * i] = k.x; w.k[2 * i + 1] = k.y;
+                w.g[2 * i] = g.x; w.g[2 * i + 1] = g.y;
+            }
+            w.beta = bs[2 * tt];
+            w.qk = bs[2 * tt + 1];
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) w.v[c] = vs[tt * DVT + cl + c];
+        };
+        auto token = [&](const Rows& w, Rows& next, int tt) {
+            if (tt + 1 < tc) read(next, tt + 1);
+            float s[2 * COLS];                     // p of the columns, then r
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                f32x2 p0 = pack2f(0.0f, 0.0f), p1 = p0, r0 = p0, r1 = p0;
+#pragma unroll
+                for (int i = 0; i < DKP / 2; i += 2) {
+                    S[c][i] = mul2f(S[c][i], w.g[i]);
+                    S[c][i + 1] = mul2f(S[c][i + 1], w.g[i + 1]);
+                    p0 = fma2f(S[c][i], w.k[i], p0);
+                    r0 = fma2f(S[c][i], w.q[i], r0);
+                    p1 = fma2f(S[c][i + 1], w.k[i + 1], p1);
+                    r1 = fma2f(S[c][i + 1], w.q[i + 1], r1);
+                }
+                s[c] = sum2f(p0) + sum2f(p1);
+                s[COLS + c] = sum2f(r0) + sum2f(r1);
+            }
+            walk_halve<2 * COLS>(s, part, P >> 1);
+            float mine_u = 0.0f;                   // u of the column whose r this lane ends with
+            const int held = part / rep;
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                const float u = w.beta * (w.v[c] - __shfl_sync(0xffffffffu, s[0], lane0 + c * rep));
+                const f32x2 uu = pack2f(u, u);
+#pragma unroll
+                for (int i = 0; i < DKP / 2; ++i) S[c][i] = fma2f(w.k[i], uu, S[c][i]);
+                if (held == COLS + c) mine_u = u;
+            }
+            if (held >= COLS && part % rep == 0) os[tt * DVT + cl + held - COLS] = fmaf(w.qk, mine_u, s[0]);
+        };
+        Rows even, odd;
+        read(even, 0);
+        for (int tt = 0; tt < tc; tt += 2) {
+            token(even, odd, tt);
+            if (tt + 1 < tc) token(odd, even, tt + 1);
+        }
+        __syncthreads();
+        for (int idx = tid; idx < tc * DVT; idx += nthreads) {
+            const int tt = idx / DVT, j = idx - tt * DVT, c = col0 + j;
+            if (c < a.dv) a.out[(size_t)(c0 + tt) * a.ldo + h * a.dv + c] = os[idx];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int i = 0; i < DKP / 2; ++i) {
+            const int kr = part * DKP + 2 * i;
+            float x, y;
+            unpack2f(S[c][i], x, y);
+            if (col + c < a.dv && kr < dk) st[(size_t)kr * a.dv + col + c] = x;
+            if (col + c < a.dv && kr + 1 < dk) st[(size_t)(kr + 1) * a.dv + col + c] = y;
+        }
+}
+
+// The same with one column a thread and a sum at a time, for few heads and requests: there a warp is alone on its scheduler, every
+// instruction of a token is waited for, and a token of one column has the fewest (one prompt of 2,048, 32 heads of 128 x 128: 1,176 us, with
+// two columns 1,359, with four 1,654; with one column and the halved sums above 1,289).
+template <int DKP>
+__global__ void __launch_bounds__(128)
+delta_walk_column_kernel(DeltaArgs a, const float* __restrict__ work, long long ldw, int P, int DVT) {
     extern __shared__ __align__(16) float sm[];
     pdl_start();
     const int r = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * DVT;
@@ -796,20 +1096,23 @@ static int launch_delta(const DeltaArgs& a, int n_reqs, cudaStream_t s);
 
 constexpr int WALK_SMEM = 64 * 1024;
 
-template <int DKP>
-static int launch_walk(const DeltaArgs& b, dim3 grid, int threads, size_t bytes, const float* work, long long ldw, int P, int dvt,
-                       cudaStream_t s) {
+template <int DKP, int COLS>
+static int launch_walk(DeltaArgs b, int n_reqs, const float* work, long long ldw, int P, cudaStream_t s) {
+    const int dvt = 128 / P * COLS;
+    int chunk = 16;
+    auto bytes = [&](int tc) { return (size_t)tc * (2 * (3 * P * (DKP + 4) + dvt + 2) + dvt) * sizeof(float); };
+    while (chunk > 4 && bytes(chunk) > WALK_SMEM) chunk >>= 1;
     static unsigned long long configured = 0;
-    if (int e = vcb_allow_dynamic_smem(delta_walk_kernel<DKP>, WALK_SMEM, &configured)) return e;
-    vcb_launch(delta_walk_kernel<DKP>, grid, threads, bytes, s, b, work, ldw, P, dvt);
+    if (int e = vcb_allow_dynamic_smem(delta_walk_kernel<DKP, COLS>, WALK_SMEM, &configured)) return e;
+    b.chunk = chunk;
+    vcb_launch(delta_walk_kernel<DKP, COLS>, dim3(n_reqs, b.H, (b.dv + dvt - 1) / dvt), 128, bytes(chunk), s, b, work, ldw, P, dvt);
     return vcb_last_error();
 }
 
 template <typename T>
 static int launch_delta_portions(const DeltaArgs& a, int n_reqs, int n_tokens, float* work, cudaStream_t s) {
-    // 8 rows of a column per thread where the key channels fill 16 lanes (keys of 128), fewer lanes for shorter keys, 16 rows
-    // for longer ones; CTAs of four warps, so that a head's columns spread over many SMs.  Measured at 16 heads of 128 x 128
-    // over 2,048 tokens: 16 rows a thread or 4 rows in CTAs of 16 warps are both slower.
+    // 8 rows of a column per thread where the key channels fill 16 lanes (keys of 128), fewer lanes for shorter keys, 16 rows for longer
+    // ones; CTAs of four warps, so that a head's columns spread over many SMs.
     const int dkp = a.dk > 256 ? 16 : 8;
     int P = 1;
     while (P * dkp < a.dk) P <<= 1;
@@ -822,12 +1125,25 @@ static int launch_delta_portions(const DeltaArgs& a, int n_reqs, int n_tokens, f
     const long long items = (long long)n_tokens * a.H;
     vcb_launch(delta_prepare_kernel<T>, dim3((unsigned)((items + 3) / 4)), 128, 0, s, a, work, ldw, n_tokens);
     if (int e = vcb_last_error()) return e;
+    // Columns a thread: four or two where the device still has two and a half warps a scheduler then (32 heads of 128 x 128, us with
+    // one / two / four: 8 prompts of together 2,048 tokens 1,093 / 704 / 645, 3 of 700 1,129 / 792 / 606, 2 of together 1,024 682 / 448 /
+    // 540, 1 of 2,048 1,176 / 1,359 / 1,654).  They need at least eight lanes a column group (the eight sums of four columns then end in
+    // lanes of their own), which keys below 64 channels leave partly idle.
+    const int lanes = P < 8 ? 8 : P;
+    const auto warps = [&](int cols) { const int w = 128 / lanes * cols; return 4LL * n_reqs * a.H * ((a.dv + w - 1) / w); };
+    const long long enough = 10LL * vcb_sm_count();
+    const int cols = warps(4) >= enough ? 4 : warps(2) >= enough ? 2 : 1;
+    if (cols == 4) return dkp == 8 ? launch_walk<8, 4>(a, n_reqs, work, ldw, lanes, s) : launch_walk<16, 4>(a, n_reqs, work, ldw, lanes, s);
+    if (cols == 2) return dkp == 8 ? launch_walk<8, 2>(a, n_reqs, work, ldw, lanes, s) : launch_walk<16, 2>(a, n_reqs, work, ldw, lanes, s);
     DeltaArgs b = a;
     b.chunk = chunk;
-    dim3 grid(n_reqs, a.H, (a.dv + dvt - 1) / dvt);
-    const int threads = dvt * P;
-    if (dkp == 8) return launch_walk<8>(b, grid, threads, bytes(chunk), work, ldw, P, dvt, s);
-    return launch_walk<16>(b, grid, threads, bytes(chunk), work, ldw, P, dvt, s);
+    const dim3 grid(n_reqs, a.H, (a.dv + dvt - 1) / dvt);
+    static unsigned long long configured[2];
+    if (int e = dkp == 8 ? vcb_allow_dynamic_smem(delta_walk_column_kernel<8>, WALK_SMEM, &configured[0])
+                         : vcb_allow_dynamic_smem(delta_walk_column_kernel<16>, WALK_SMEM, &configured[1])) return e;
+    if (dkp == 8) vcb_launch(delta_walk_column_kernel<8>, grid, dvt * P, bytes(chunk), s, b, (const float*)work, ldw, P, dvt);
+    else vcb_launch(delta_walk_column_kernel<16>, grid, dvt * P, bytes(chunk), s, b, (const float*)work, ldw, P, dvt);
+    return vcb_last_error();
 }
 
 template <typename T>
