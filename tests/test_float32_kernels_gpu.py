@@ -117,3 +117,22 @@ def test_attention_rows(ops, dtype, nh, nkv, d, page, planes, window, sink):
         tol = 2e-5 if dtype == torch.float32 else 2e-5 + 2.0 ** -8
         assert bool(((out.view(len(pos), nh, d).double() - want).abs() <= tol * size.clamp(min=1.0)).all())
     ops.check_status()
+
+
+@pytest.mark.parametrize("nh,nkv,d,window", [(4, 4, 32, 0), (14, 2, 128, 0), (8, 1, 256, 90)])
+def test_attention_rows_do_not_depend_on_the_call(ops, nh, nkv, d, window):
+    """A token alone (a warp per part of its keys) and among many (two and four warps, and one, walk the parts) has the same bits, with keys of one
+    part, of a few and of eight."""
+    dev = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()  # noqa: E731
+    q, cache, rows, pos, req, bt = _attention_case(nh, [1, 63, 64, 65, 200, 530], [1] * 6, nh, nkv, d, 16, 2, torch.float32)
+
+    def run(times):
+        at = np.tile(np.arange(6), times)
+        out = torch.empty(len(at), nh * d, device="cuda")
+        ops.attention_simt(q.view(6, -1)[dev(at)].contiguous(), cache, out, dev(pos[at]), dev(req[at]), dev(bt), num_heads=nh, num_kv_heads=nkv, head_dim=d,
+                           page_size=16, window=window, scale=d ** -0.5)
+        return out.view(times, 6, -1)
+    alone = run(1)
+    for times in (20, 40, 90, 150, 400):
+        assert torch.equal(run(times), alone.expand(times, -1, -1))
+    ops.check_status()

@@ -121,12 +121,14 @@ __global__ void attention_simt_kernel(AttnArgs a) {
 // walks four keys at a time, so that a key's row is read once for all of them, 16 bytes a lane.  LPR lanes hold a row (CH
 // 16-byte pieces each; 32 / LPR rows are read side by side).  The products of a lane's piece with GH queries and four keys are
 // summed over the row's lanes by halving: each exchange adds two lanes' values and leaves each lane half of them, 31
-// exchanges for 32 sums where a butterfly per sum takes 160.  `split` warps share one token's keys where there are too few tokens to
-// fill the device, and join their sums in shared memory.
+// exchanges for 32 sums where a butterfly per sum takes 160.  A token's keys are walked in parts, one per ATT_PART_KEYS keys up to eight, every
+// part with a softmax of its own; the parts are joined in their order.  Where there are too few tokens to fill the device `split` warps
+// take parts side by side, else one warp walks them one after another: the sums are the same, so a token's bits do not depend on the batch.
 // The kernel above reads 32 rows 4 bytes at a time, a sector each, once per head: at 28 heads on 4 kv heads of 128, float32, it took
-// 1,404 us for one token after 2,048, 125 us for three after 170, 12.2 ms for a prompt of 2,048; this one takes 91, 17 and 2.6.  Bound by
+// 1,404 us for one token after 2,048, 125 us for three after 170, 12.2 ms for a prompt of 2,048; this one takes 88, 16 and 2.7.  Bound by
 // the latency of a round (a row's loads, five exchanges, two exponentials): a CTA of 8 warps is all that 200 registers a thread allow.
 #define ATT_ROW_WARPS 8
+#define ATT_PART_KEYS 32            // with 64: 113, 25 and, the reads not running ahead across parts, 3.5
 
 template <typename T> struct RowPiece;
 template <> struct RowPiece<float> {
@@ -165,6 +167,11 @@ __device__ __forceinline__ void sum_over_lanes(float* s, int lane) {
     }
 }
 
+// What a part's sums and those before it are multiplied by when both are taken to the larger of their maxima (one of them is finite, or both
+// sums are zeros).
+__device__ __forceinline__ float part_factor(float m, float m_new) { return m > -INFINITY ? expf(m - m_new) : 0.0f; }
+__device__ __forceinline__ float part_join(float before, float f, float part, float g) { return fmaf(part, g, __fmul_rn(before, f)); }
+
 template <typename T, int LPR, int CH, int GH>
 __global__ void __launch_bounds__(ATT_ROW_WARPS * 32)
 attention_rows_kernel(AttnArgs a, int split) {
@@ -178,8 +185,8 @@ attention_rows_kernel(AttnArgs a, int split) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane / LPR, rl = lane % LPR;
     const int group = a.nh / a.nkv, chunks = (group + GH - 1) / GH;
     const long long items = (long long)a.n_tokens * a.nkv * chunks;
+    const int sub = warp % split;
     const long long item = (long long)blockIdx.x * (ATT_ROW_WARPS / split) + warp / split;      // neighbours: tokens of the same kv head
-    const int part = warp % split;
     const bool live = item < items;
     const int t = live ? (int)(item % a.n_tokens) : 0, gc = live ? (int)(item / a.n_tokens) : 0, g = gc / chunks, h0 = (gc % chunks) * GH;
     const int heads = min(GH, group - h0);                 // of this warp; the sums beyond them are zero and not stored
@@ -204,7 +211,7 @@ attention_rows_kernel(AttnArgs a, int split) {
         return swizzled ? base[c] + slot * PER_PLANE + ((chunk[c] ^ (slot & 7)) * PER_CHUNK) + within[c] : base[c] + slot * a.d;
     };
 
-    float4 q[GH][CH], o[GH][CH];
+    float4 q[GH][CH], o[GH][CH];                           // o: of one part, at the end of the row
 #pragma unroll
     for (int h = 0; h < GH; ++h)
 #pragma unroll
@@ -212,12 +219,13 @@ attention_rows_kernel(AttnArgs a, int split) {
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (live && h < heads && has[c]) v = RowPiece<T>::load((const T*)a.q + ((size_t)t * a.nh + g * group + h0 + h) * a.d + (c * LPR + rl) * 4);
             q[h][c] = make_float4(v.x * a.scale, v.y * a.scale, v.z * a.scale, v.w * a.scale);
-            o[h][c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     // the (head, key) whose score this lane ends with
     const int mine = rl / REP, my_head = mine / KPG, my_key = rg * KPG + mine % KPG;
-    float m = -INFINITY, l = 0.0f;                         // of my_head, over the keys of all lanes
+    float m, l;                                            // of my_head, over the part's keys of all lanes
     const int kstart = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+    const int parts = max(1, min(ATT_ROW_WARPS, (pos - kstart + ATT_PART_KEYS) / ATT_PART_KEYS));
+    const int stride = 4 * parts, steps = (pos - kstart + stride) / stride;      // of four keys, per part; the last ones of a part may be past pos
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 
     // Rows are read a round ahead of their use, pages' numbers two: a round waits for neither (unpipelined it took 3,500 cycles).
@@ -248,95 +256,12 @@ attention_rows_kernel(AttnArgs a, int split) {
             }
         }
     };
-    const int first = kstart + 4 * part, stride = 4 * split;
-    int page_now, slot_now, page_next, slot_next;
-    float4 k[KPG][CH], v[KPG][CH], k_next[KPG][CH], v_next[KPG][CH];
-    find(first, page_now, slot_now);
-    find(first + stride, page_next, slot_next);
-    fetch(page_now, slot_now, k, v);
-    for (int kb = first; kb <= pos; kb += stride) {
-        const int page_of = page_now;
-        fetch(page_next, slot_next, k_next, v_next);
-        page_now = page_next;
-        find(kb + 2 * stride, page_next, slot_next);
-        float s[NV];
-#pragma unroll
-        for (int h = 0; h < GH; ++h)
-#pragma unroll
-            for (int kk = 0; kk < KPG; ++kk) {
-                float x = 0.0f;
-#pragma unroll
-                for (int c = 0; c < CH; ++c) {
-                    x = fmaf(q[h][c].x, k[kk][c].x, x);
-                    x = fmaf(q[h][c].y, k[kk][c].y, x);
-                    x = fmaf(q[h][c].z, k[kk][c].z, x);
-                    x = fmaf(q[h][c].w, k[kk][c].w, x);
-                }
-                s[h * KPG + kk] = x;
-            }
-        sum_over_lanes<NV, LPR / 2>(s, rl);                // lane rl ends with sum rl / REP
-        const bool valid = __shfl_sync(0xffffffffu, page_of, my_key) >= 0;
-        const float score = valid ? s[0] : -INFINITY;
-        // over the four keys: those of a row group differ in the lane's bits above REP, the groups in the bits above LPR
-        float top = score;
-#pragma unroll
-        for (int bit = REP; bit < REP * KPG; bit <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, bit));
-#pragma unroll
-        for (int bit = LPR; bit < 32; bit <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, bit));
-        const float m_new = fmaxf(m, top);
-        const float p = valid ? expf(score - m_new) : 0.0f;
-        float sum = p;
-#pragma unroll
-        for (int bit = REP; bit < REP * KPG; bit <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, bit);
-#pragma unroll
-        for (int bit = LPR; bit < 32; bit <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, bit);
-        const bool moved = m_new > m;
-        if (__any_sync(0xffffffffu, moved)) {
-            const float corr = moved ? expf(m - m_new) : 1.0f;
-            l *= corr;
-#pragma unroll
-            for (int h = 0; h < GH; ++h) {
-                const float f = __shfl_sync(0xffffffffu, corr, h * KPG * REP);
-#pragma unroll
-                for (int c = 0; c < CH; ++c) { o[h][c].x *= f; o[h][c].y *= f; o[h][c].z *= f; o[h][c].w *= f; }
-            }
-            m = m_new;
-        }
-        l += sum;
-        __syncwarp();
-        if (rl % REP == 0) p_all[warp][rg * NV + mine] = p;
-        __syncwarp();
-#pragma unroll
-        for (int h = 0; h < GH; ++h)
-#pragma unroll
-            for (int kk = 0; kk < KPG; ++kk) {
-                const float w = p_all[warp][rg * NV + h * KPG + kk];
-#pragma unroll
-                for (int c = 0; c < CH; ++c) {
-                    o[h][c].x = fmaf(w, v[kk][c].x, o[h][c].x);
-                    o[h][c].y = fmaf(w, v[kk][c].y, o[h][c].y);
-                    o[h][c].z = fmaf(w, v[kk][c].z, o[h][c].z);
-                    o[h][c].w = fmaf(w, v[kk][c].w, o[h][c].w);
-                }
-            }
-#pragma unroll
-        for (int kk = 0; kk < KPG; ++kk)
-#pragma unroll
-            for (int c = 0; c < CH; ++c) { k[kk][c] = k_next[kk][c]; v[kk][c] = v_next[kk][c]; }
-    }
-    // the row groups' sums (they share the maxima)
-#pragma unroll
-    for (int bit = LPR; bit < 32; bit <<= 1)
-#pragma unroll
-        for (int h = 0; h < GH; ++h)
-#pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                o[h][c].x += __shfl_xor_sync(0xffffffffu, o[h][c].x, bit);
-                o[h][c].y += __shfl_xor_sync(0xffffffffu, o[h][c].y, bit);
-                o[h][c].z += __shfl_xor_sync(0xffffffffu, o[h][c].z, bit);
-                o[h][c].w += __shfl_xor_sync(0xffffffffu, o[h][c].w, bit);
-            }
-    if (split > 1) {
+    // part round + sub of every round; joined in their order by the group's first warp, whose slot of shared memory keeps the sums between rounds
+    auto group_barrier = [&]() {
+        if (split == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / split), "r"(32 * split) : "memory");
+    };
+    auto leave = [&]() {
         if (rg == 0) {
 #pragma unroll
             for (int h = 0; h < GH; ++h)
@@ -344,36 +269,142 @@ attention_rows_kernel(AttnArgs a, int split) {
                 for (int c = 0; c < CH; ++c) *reinterpret_cast<float4*>(&join_o[warp][h][(c * LPR + rl) * 4]) = o[h][c];
             if (mine % KPG == 0 && rl % REP == 0) { join_ml[warp][0][my_head] = m; join_ml[warp][1][my_head] = l; }
         }
-        __syncthreads();
-        if (part != 0) return;
-        // a warp that had no key left m = -inf, l = 0 and zeros
-        float mj = -INFINITY;
-        for (int w = 0; w < split; ++w) mj = fmaxf(mj, join_ml[warp + w][0][my_head]);
-        l = 0.0f;
-        for (int w = 0; w < split; ++w) {
-            const float mw = join_ml[warp + w][0][my_head];
-            l += mw > -INFINITY ? join_ml[warp + w][1][my_head] * expf(mw - mj) : 0.0f;
-        }
+    };
+    auto join = [&](int w, bool first_is_slot) {           // the sums before and a part: slot w and the registers, or the other way round
+        const float ms = join_ml[w][0][my_head], ls = join_ml[w][1][my_head], mj = fmaxf(m, ms);
+        const float fs = part_factor(ms, mj), fr = part_factor(m, mj);
+        l = first_is_slot ? part_join(ls, fs, l, fr) : part_join(l, fr, ls, fs);
         m = mj;
 #pragma unroll
         for (int h = 0; h < GH; ++h) {
+            const float hs = __shfl_sync(0xffffffffu, fs, h * KPG * REP), hr = __shfl_sync(0xffffffffu, fr, h * KPG * REP);
 #pragma unroll
-            for (int c = 0; c < CH; ++c) o[h][c] = zero;
-            float mh = -INFINITY;
-            for (int w = 0; w < split; ++w) mh = fmaxf(mh, join_ml[warp + w][0][h]);
-            for (int w = 0; w < split; ++w) {
-                const float mw = join_ml[warp + w][0][h];
-                if (!(mw > -INFINITY)) continue;
-                const float f = expf(mw - mh);
-#pragma unroll
-                for (int c = 0; c < CH; ++c) {
-                    const float4 x = *reinterpret_cast<const float4*>(&join_o[warp + w][h][(c * LPR + rl) * 4]);
-                    o[h][c].x = fmaf(f, x.x, o[h][c].x); o[h][c].y = fmaf(f, x.y, o[h][c].y);
-                    o[h][c].z = fmaf(f, x.z, o[h][c].z); o[h][c].w = fmaf(f, x.w, o[h][c].w);
-                }
+            for (int c = 0; c < CH; ++c) {
+                const float4 x = *reinterpret_cast<const float4*>(&join_o[w][h][(c * LPR + rl) * 4]);
+                if (first_is_slot)
+                    o[h][c] = make_float4(part_join(x.x, hs, o[h][c].x, hr), part_join(x.y, hs, o[h][c].y, hr), part_join(x.z, hs, o[h][c].z, hr),
+                                          part_join(x.w, hs, o[h][c].w, hr));
+                else
+                    o[h][c] = make_float4(part_join(o[h][c].x, hr, x.x, hs), part_join(o[h][c].y, hr, x.y, hs), part_join(o[h][c].z, hr, x.z, hs),
+                                          part_join(o[h][c].w, hr, x.w, hs));
             }
         }
+    };
+    // what is found next: four keys of a part, then the next part of this warp, so that the reads run ahead across parts
+    int find_part = sub, find_step = 0;
+    auto find_next = [&](int& page_of, int& slot_of) {
+        find(find_part < parts ? kstart + 4 * find_part + find_step * stride : pos + 1, page_of, slot_of);
+        if (++find_step == steps) {
+            find_step = 0;
+            find_part += split;
+        }
+    };
+    int page_now, slot_now, page_next, slot_next;
+    float4 k[KPG][CH], v[KPG][CH], k_next[KPG][CH], v_next[KPG][CH];
+    find_next(page_now, slot_now);
+    find_next(page_next, slot_next);
+    fetch(page_now, slot_now, k, v);
+    for (int round = 0; round < parts; round += split) {
+        m = -INFINITY;
+        l = 0.0f;
+#pragma unroll
+        for (int h = 0; h < GH; ++h)
+#pragma unroll
+            for (int c = 0; c < CH; ++c) o[h][c] = zero;
+        for (int step = round + sub < parts ? 0 : steps; step < steps; ++step) {
+            const int page_of = page_now;
+            fetch(page_next, slot_next, k_next, v_next);
+            page_now = page_next;
+            find_next(page_next, slot_next);
+            float s[NV];
+#pragma unroll
+            for (int h = 0; h < GH; ++h)
+#pragma unroll
+                for (int kk = 0; kk < KPG; ++kk) {
+                    float x = 0.0f;
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) {
+                        x = fmaf(q[h][c].x, k[kk][c].x, x);
+                        x = fmaf(q[h][c].y, k[kk][c].y, x);
+                        x = fmaf(q[h][c].z, k[kk][c].z, x);
+                        x = fmaf(q[h][c].w, k[kk][c].w, x);
+                    }
+                    s[h * KPG + kk] = x;
+                }
+            sum_over_lanes<NV, LPR / 2>(s, rl);                // lane rl ends with sum rl / REP
+            const bool valid = __shfl_sync(0xffffffffu, page_of, my_key) >= 0;
+            const float score = valid ? s[0] : -INFINITY;
+            // over the four keys: those of a row group differ in the lane's bits above REP, the groups in the bits above LPR
+            float top = score;
+#pragma unroll
+            for (int bit = REP; bit < REP * KPG; bit <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, bit));
+#pragma unroll
+            for (int bit = LPR; bit < 32; bit <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, bit));
+            const float m_new = fmaxf(m, top);
+            const float p = valid ? expf(score - m_new) : 0.0f;
+            float sum = p;
+#pragma unroll
+            for (int bit = REP; bit < REP * KPG; bit <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, bit);
+#pragma unroll
+            for (int bit = LPR; bit < 32; bit <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, bit);
+            const bool moved = m_new > m;
+            if (__any_sync(0xffffffffu, moved)) {
+                const float corr = moved ? expf(m - m_new) : 1.0f;
+                l *= corr;
+#pragma unroll
+                for (int h = 0; h < GH; ++h) {
+                    const float f = __shfl_sync(0xffffffffu, corr, h * KPG * REP);
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) { o[h][c].x *= f; o[h][c].y *= f; o[h][c].z *= f; o[h][c].w *= f; }
+                }
+                m = m_new;
+            }
+            l += sum;
+            __syncwarp();
+            if (rl % REP == 0) p_all[warp][rg * NV + mine] = p;
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < GH; ++h)
+#pragma unroll
+                for (int kk = 0; kk < KPG; ++kk) {
+                    const float w = p_all[warp][rg * NV + h * KPG + kk];
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) {
+                        o[h][c].x = fmaf(w, v[kk][c].x, o[h][c].x);
+                        o[h][c].y = fmaf(w, v[kk][c].y, o[h][c].y);
+                        o[h][c].z = fmaf(w, v[kk][c].z, o[h][c].z);
+                        o[h][c].w = fmaf(w, v[kk][c].w, o[h][c].w);
+                    }
+                }
+#pragma unroll
+            for (int kk = 0; kk < KPG; ++kk)
+#pragma unroll
+                for (int c = 0; c < CH; ++c) { k[kk][c] = k_next[kk][c]; v[kk][c] = v_next[kk][c]; }
+        }
+        // the row groups' sums (they share the maxima)
+#pragma unroll
+        for (int bit = LPR; bit < 32; bit <<= 1)
+#pragma unroll
+            for (int h = 0; h < GH; ++h)
+#pragma unroll
+                for (int c = 0; c < CH; ++c) {
+                    o[h][c].x += __shfl_xor_sync(0xffffffffu, o[h][c].x, bit);
+                    o[h][c].y += __shfl_xor_sync(0xffffffffu, o[h][c].y, bit);
+                    o[h][c].z += __shfl_xor_sync(0xffffffffu, o[h][c].z, bit);
+                    o[h][c].w += __shfl_xor_sync(0xffffffffu, o[h][c].w, bit);
+                }
+        if (parts == 1) break;
+        if (sub > 0) leave();                              // nothing but -inf and zeros where the parts are used up
+        group_barrier();
+        if (sub == 0) {
+            if (round > 0) join(warp, true);
+            for (int w = 1; w < split && round + w < parts; ++w) join(warp + w, false);
+            __syncwarp();                                  // read before it is written
+            if (round + split < parts) leave();
+        }
+        if (round + split < parts) group_barrier();
     }
+    if (sub > 0) return;
     if (!live) return;
     float inv = 1.0f / l;
     if (a.sink) {
