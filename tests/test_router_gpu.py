@@ -1,0 +1,44 @@
+"""Router logits of few tokens (a CTA per output), of many (two, five and eight outputs a warp) and of rows that 4-element pieces do not cover, and the
+choices' rows joined four elements at a time and one at a time; against 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,width,outs", [(1, 4, 3), (8, 1028, 33), (9, 2052, 16), (64, 4096, 40), (65, 4096, 16), (65, 1028, 17), (71, 132, 41), (200, 260, 130),
+                                          (3, 1030, 9), (70, 1030, 9)])
+def test_logits_and_choice(n, width, outs, dtype):
+    from vllm_cpp_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(n + width)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    top = min(4, outs)
+    h = rnd(n, width + 4).to(dtype)[:, :width]
+    w = rnd(outs, width) / width ** 0.5
+    ids, weights = torch.empty(n, top, dtype=torch.int32, device="cuda"), torch.empty(n, top, device="cuda")
+    logits = torch.full((n, outs), 9.0, device="cuda")
+    ops.moe_router(h, w, None, ids, weights, logits, score="sigmoid")
+    want = h.double() @ w.double().T
+    # float32 sums of `width` products of size 1 / sqrt(width), in at most 32 + 8 + width / 256 steps
+    assert bool(((logits.double() - want).abs() <= 1e-5).all())
+    assert torch.equal(ids.long(), logits.topk(top, dim=1).indices)
+    assert bool(((weights.double() - torch.sigmoid(logits.double()).gather(1, ids.long())).abs() <= 1e-6).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,width,top", [(1, 4, 1), (5, 1028, 3), (7, 1024, 4), (9, 132, 5), (3, 4096, 9), (6, 130, 3)])
+def test_combine(n, width, top, dtype):
+    from vllm_cpp_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(n + width)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    y, h, add, weights = rnd(n * top, width), rnd(n, width + 4).to(dtype)[:, :width], rnd(n, width).to(dtype), rnd(n, top)
+    pos = torch.randperm(n * top, device="cuda", generator=gen).to(torch.int32).view(n, top)
+    pos[rnd(n, top) > 1.0] = -1
+    rows = torch.where((pos >= 0)[..., None], y.double()[pos.clamp(min=0).long()], h.double()[:, None, :])
+    for w, more in ((weights, add), (None, None), (weights, None)):
+        out = torch.full((n, width), 9.0, dtype=dtype, device="cuda")
+        ops.moe_combine(y, h, pos, w, out, more)
+        want = (rows * (w.double()[..., None] if w is not None else 1.0)).sum(1) + (more.double() if more is not None else 0.0)
+        # top + 1 float32 additions of numbers up to 5, and the stored type's rounding
+        assert bool(((out.double() - want).abs() <= 1e-5 * (1 + want.abs()) + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)).all())

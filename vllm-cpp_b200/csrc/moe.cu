@@ -24,9 +24,12 @@
 #include <cuda.h>
 
 // ------------------------------------------------------------------------------------------- router
-// Two kernels.  Logits: a CTA takes RT_TOK tokens and eight router outputs, a warp per output: the tokens' rows pass
-// through shared memory in slabs (as float), a row of the float32 router matrix is read once for the CTA's tokens
-// with 16-byte loads.  Selection: a warp per token does the softmax over all outputs, adds the correction and
+// Logits, then selection.  Logits: where 4-element pieces cover the rows, two kernels.  Few tokens: a CTA per router output and eight
+// tokens, its 256 threads split the row, so that a row of 4,096 is four independent loads of the matrix and 32 of the tokens a thread
+// (8 tokens, 33 outputs of 4,096: 6.5 us).  Many: eight tokens a CTA, a warp four to eight outputs, so that a
+// token's piece is read for several outputs and a matrix's piece for eight tokens (2,048 tokens: 36 us; 16 calls of 8 tokens and two of
+// 2,048 took 398 us with a warp per output and four tokens in shared memory, now 176).  Else a CTA takes RT_TOK tokens and eight router outputs, a warp per output: the tokens' rows pass
+// through shared memory in slabs (as float).  Selection: a warp per token does the softmax over all outputs, adds the correction and
 // picks the `top` largest (the lower index wins among equals); the plain scores of the chosen are the weights.
 #define RT_TOK 4
 #define RT_SLAB 2048
@@ -85,6 +88,102 @@ moe_router_logits_kernel(const T* __restrict__ h, long long ldh, const float* __
         const float v = warp_sum(acc[t]);
         if (lane == 0 && t0 + t < n_tokens) logits[(size_t)(t0 + t) * n_out + e] = v;
     }
+}
+
+template <typename T> __device__ __forceinline__ float4 router_piece(const T* p);
+template <> __device__ __forceinline__ float4 router_piece<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 router_piece<__nv_bfloat16>(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float dot4(float4 a, float4 b, float c) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c)))); }
+
+constexpr int RT_FEW_TOK = 8;
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_router_few_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr, float* __restrict__ logits, int n_tokens, int width, int n_out) {
+    __shared__ float sums[8][RT_FEW_TOK];
+    const int t0 = blockIdx.x * RT_FEW_TOK, e = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float* w = wr + (size_t)e * width;
+    float acc[RT_FEW_TOK];
+#pragma unroll
+    for (int t = 0; t < RT_FEW_TOK; ++t) acc[t] = 0.0f;
+    pdl_start();
+    for (int k = threadIdx.x * 4; k < width; k += 2048) {
+        const bool second = k + 1024 < width;
+        const float4 a = router_piece<float>(w + k), b = second ? router_piece<float>(w + k + 1024) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 x[RT_FEW_TOK], y[RT_FEW_TOK];
+#pragma unroll
+        for (int t = 0; t < RT_FEW_TOK; ++t) {
+            const T* row = h + (size_t)min(t0 + t, n_tokens - 1) * ldh;        // rows beyond the last repeat it; they are not stored
+            x[t] = router_piece<T>(row + k);
+            y[t] = router_piece<T>(row + (second ? k + 1024 : k));
+        }
+#pragma unroll
+        for (int t = 0; t < RT_FEW_TOK; ++t) acc[t] = dot4(y[t], b, dot4(x[t], a, acc[t]));
+    }
+#pragma unroll
+    for (int t = 0; t < RT_FEW_TOK; ++t) {
+        const float v = warp_sum(acc[t]);
+        if (lane == 0) sums[warp][t] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < RT_FEW_TOK && t0 + (int)threadIdx.x < n_tokens) {
+        float v = 0.0f;
+        for (int q = 0; q < 8; ++q) v += sums[q][threadIdx.x];
+        logits[(size_t)(t0 + threadIdx.x) * n_out + e] = v;
+    }
+}
+
+template <typename T, int OUTS>
+__global__ void __launch_bounds__(256)
+moe_router_many_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr, float* __restrict__ logits, int n_tokens, int width, int n_out) {
+    constexpr int TOK = 8;
+    const int t0 = blockIdx.x * TOK, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int e0 = (blockIdx.y * 8 + warp) * OUTS;
+    pdl_start();
+    if (e0 >= n_out) return;
+    float acc[OUTS][TOK];
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o)
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) acc[o][t] = 0.0f;
+    for (int k = lane * 4; k < width; k += 128) {
+        float4 x[TOK];
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) x[t] = router_piece<T>(h + (size_t)min(t0 + t, n_tokens - 1) * ldh + k);
+#pragma unroll
+        for (int o = 0; o < OUTS; ++o) {
+            const float4 w = router_piece<float>(wr + (size_t)min(e0 + o, n_out - 1) * width + k);
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) acc[o][t] = dot4(x[t], w, acc[o][t]);
+        }
+    }
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o)
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) {
+            const float v = warp_sum(acc[o][t]);
+            if (lane == 0 && t0 + t < n_tokens && e0 + o < n_out) logits[(size_t)(t0 + t) * n_out + e0 + o] = v;
+        }
+}
+
+template <typename T>
+static void launch_router_logits(const T* h, long long ldh, const float* wr, float* logits, int n_tokens, int width, int n_out, cudaStream_t s) {
+    if ((width & 3) == 0 && (ldh & 3) == 0 && (((uintptr_t)wr) & 15) == 0 && (((uintptr_t)h) & (4 * sizeof(T) - 1)) == 0) {
+        // few: as long as the CTAs per output leave the device room
+        if (n_tokens <= 64 && n_out <= 65535) {
+            vcb_launch(moe_router_few_kernel<T>, dim3((n_tokens + RT_FEW_TOK - 1) / RT_FEW_TOK, n_out), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
+            return;
+        }
+        const int blocks = (n_tokens + 7) / 8;
+        if (n_out <= 16) vcb_launch(moe_router_many_kernel<T, 2>, dim3(blocks, (n_out + 15) / 16), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
+        else if (n_out <= 40) vcb_launch(moe_router_many_kernel<T, 5>, dim3(blocks, (n_out + 39) / 40), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
+        else vcb_launch(moe_router_many_kernel<T, 8>, dim3(blocks, (n_out + 63) / 64), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
+        return;
+    }
+    vcb_launch(moe_router_logits_kernel<T>, dim3((n_tokens + RT_TOK - 1) / RT_TOK, (n_out + 7) / 8), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
 }
 
 // How the scores are made and used (the fields a design does not have stay at their neutral values).
@@ -201,10 +300,8 @@ VCB_EXPORT int vcb_moe_router_biased(const void* h, long long ldh, const float* 
     const size_t smem = (size_t)4 * (2 * n_out + n_groups) * sizeof(float);
     if (smem > 48 * 1024 || (n_out + 7) / 8 > 65535) return VCB_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid((n_tokens + RT_TOK - 1) / RT_TOK, (n_out + 7) / 8);
-    if (dtype == VCB_F32) vcb_launch(moe_router_logits_kernel<float>, grid, 256, 0, s, (const float*)h, ldh, wr, logits, n_tokens, width, n_out);
-    else if (dtype == VCB_BF16)
-        vcb_launch(moe_router_logits_kernel<__nv_bfloat16>, grid, 256, 0, s, (const __nv_bfloat16*)h, ldh, wr, logits, n_tokens, width, n_out);
+    if (dtype == VCB_F32) launch_router_logits<float>((const float*)h, ldh, wr, logits, n_tokens, width, n_out, s);
+    else if (dtype == VCB_BF16) launch_router_logits<__nv_bfloat16>((const __nv_bfloat16*)h, ldh, wr, logits, n_tokens, width, n_out, s);
     else return VCB_ERR_BAD_ARG;
     RouteRule rule{score_fn, n_groups, keep_groups, group_top, normalize, sum_eps, scale};
     vcb_launch(moe_router_select_kernel, (n_tokens + 3) / 4, 128, smem, s, (const float*)logits, logit_bias, correction, ids, wts, n_tokens, n_out, top, rule);
@@ -847,16 +944,62 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const T* __restr
     }
 }
 
+// The same four elements at a time where the rows allow 4-element pieces: the choices' rows are loaded before the first is used (four at a
+// time), and a token's row is spread over CTAs of 256 pieces.  16 calls of 8 tokens and two of
+// 2,048, 4 choices, width 4,096: 347 us one element at a time (each waited for its choice's number and then its row), now 109.
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_combine_vec_kernel(const float* __restrict__ y, const T* __restrict__ h, long long ldh, const int* __restrict__ pos, const float* __restrict__ wts,
+                       T* __restrict__ out, int width, int top, const T* __restrict__ add, long long lda) {
+    pdl_start();
+    const int t = blockIdx.x, i = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (i >= width) return;
+    float4 acc = add ? router_piece<T>(add + (size_t)t * lda + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int k0 = 0; k0 < top; k0 += 4) {
+        int p[4];
+        float w[4];
+        float4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int at = t * top + min(k0 + k, top - 1);
+            p[k] = pos[at];
+            w[k] = wts ? wts[at] : 1.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = p[k] >= 0 ? router_piece<float>(y + (size_t)p[k] * width + i) : router_piece<T>(h + (size_t)t * ldh + i);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k0 + k < top) acc = make_float4(fmaf(w[k], v[k].x, acc.x), fmaf(w[k], v[k].y, acc.y), fmaf(w[k], v[k].z, acc.z), fmaf(w[k], v[k].w, acc.w));
+    }
+    T* o = out + (size_t)t * width + i;
+    if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(o) = acc;
+    } else {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(acc.x, acc.y), b = __floats2bfloat162_rn(acc.z, acc.w);
+        *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+}
+
+template <typename T>
+static void launch_combine(const float* y, const T* h, long long ldh, const int* pos, const float* wts, T* out, int n_tokens, int width, int top, const T* add,
+                           long long lda, cudaStream_t s) {
+    const uintptr_t rows = (uintptr_t)h | (uintptr_t)out | (uintptr_t)add;
+    if ((width & 3) == 0 && ((ldh | lda) & 3) == 0 && (((uintptr_t)y) & 15) == 0 && (rows & (4 * sizeof(T) - 1)) == 0 && (width + 1023) / 1024 <= 65535 &&
+        (long long)n_tokens * top <= 0x7fffffffLL) {
+        vcb_launch(moe_combine_vec_kernel<T>, dim3(n_tokens, (width + 1023) / 1024), 256, 0, s, y, h, ldh, pos, wts, out, width, top, add, lda);
+        return;
+    }
+    vcb_launch(moe_combine_kernel<T>, n_tokens, width >= 1024 ? 256 : 128, 0, s, y, h, ldh, pos, wts, out, width, top, add, lda);
+}
+
 VCB_EXPORT int vcb_moe_combine_add(const float* y, const void* h, long long ldh, const int* pos, const float* wts, void* out,
                                    int n_tokens, int width, int top, const void* add, long long lda, int dtype, void* stream) {
     if (n_tokens <= 0) return 0;
     if (!y || !h || !pos || !out || width <= 0 || top <= 0) return VCB_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    const int threads = width >= 1024 ? 256 : 128;
-    if (dtype == VCB_F32) vcb_launch(moe_combine_kernel<float>, n_tokens, threads, 0, s, y, (const float*)h, ldh, pos, wts, (float*)out, width, top, (const float*)add, lda);
+    if (dtype == VCB_F32) launch_combine<float>(y, (const float*)h, ldh, pos, wts, (float*)out, n_tokens, width, top, (const float*)add, lda, s);
     else if (dtype == VCB_BF16)
-        vcb_launch(moe_combine_kernel<__nv_bfloat16>, n_tokens, threads, 0, s, y, (const __nv_bfloat16*)h, ldh, pos, wts,
-                   (__nv_bfloat16*)out, width, top, (const __nv_bfloat16*)add, lda);
+        launch_combine<__nv_bfloat16>(y, (const __nv_bfloat16*)h, ldh, pos, wts, (__nv_bfloat16*)out, n_tokens, width, top, (const __nv_bfloat16*)add, lda, s);
     else return VCB_ERR_BAD_ARG;
     return vcb_last_error();
 }
