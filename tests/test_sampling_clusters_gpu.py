@@ -75,6 +75,7 @@ def test_whole_rows(vocab):
     ops.sample(logits, dev(np.zeros(8)), dev(np.zeros(8)), out)
     assert out.cpu().numpy().tolist() == [int(np.argmax(r)) for r in x]
     for u in (0.0, 0.123, 0.5, 0.875, 0.99999994):
+        out.fill_(-7)
         ops.sample(logits, dev(np.ones(8)), dev(np.full(8, u)), out)
         for r, g in enumerate(out.cpu().numpy()):
             e = np.exp(x[r].astype(np.float64) - x[r].max())
@@ -82,6 +83,25 @@ def test_whole_rows(vocab):
             # sums of up to 8 x 16 slabs of float32 sums
             assert 0 <= g < vocab and (c[g - 1] if g else 0.0) - 2e-5 * c[-1] <= u * c[-1] <= c[g] + 2e-5 * c[-1], (vocab, u, r, g)
             assert e[g] > 0
+
+
+# slabs with ids, of a run's 16: 3, 15, 14, 15, all
+@pytest.mark.parametrize("vocab", [384, 1800, 100352, 152064, 65536])
+def test_every_draw_has_an_id(vocab):
+    """The largest uniform number that 24 bits give: the draw lies within the last place of the row's sum, in whichever order that was added up."""
+    from vllm_cpp_b200.csrc import ops
+    rows = 512
+    gen = torch.Generator(device="cuda").manual_seed(vocab)
+    ones, u = torch.ones(rows, device="cuda"), torch.full((rows,), 1.0 - 2.0 ** -24, device="cuda")
+    for _ in range(4):
+        logits = torch.randn(rows, vocab, device="cuda", generator=gen)
+        out = torch.full((rows,), -7, dtype=torch.int32, device="cuda")
+        ops.sample(logits, ones, u, out)
+        assert int(out.min()) >= 0 and int(out.max()) < vocab
+        # what lies behind the id drawn is at most the roundings of the sums (as in test_whole_rows)
+        e = torch.softmax(logits.double(), dim=1)
+        behind = 1.0 - e.cumsum(1).gather(1, out.long()[:, None])
+        assert bool((behind <= 2e-5).all())
 
 
 @pytest.mark.parametrize("vocab", [997, 70001])

@@ -200,7 +200,9 @@ sample_row(const float* __restrict__ logits, int ld, int vocab, const float* __r
             if (lane >= o) w += y;
         }
         scratch[lane] = w;                 // inclusive sums of the slabs
-        if (lane == nwarps - 1) cta_sum = w;
+        // The run's sum is that of its last slab with ids: an empty slab behind it adds nothing, but its sum is another tree of the same
+        // numbers and may be a unit in the last place larger, and a draw between the two would lie in no slab.
+        if (lane == (last > first ? (last - first - 1) / slab : 0)) cta_sum = w;
     }
     if (threadIdx.x == 0) winner = nwarps;
     cluster.sync();
@@ -220,7 +222,7 @@ sample_row(const float* __restrict__ logits, int ld, int vocab, const float* __r
     const float incl = before_cta + scratch[warp];
     if (lane == 0 && hi > lo && target < incl) atomicMin(&winner, warp);
     __syncthreads();
-    if (warp != winner) return;                            // the last slab that has ids ends at the run's sum, so there is one
+    if (warp != winner) return;                            // there is one: the last slab that has ids ends at the run's sum
     float c = incl - local;                      // the sum before this slab
     int tok = hi - 1;                            // if rounding keeps the walk's sums below the draw: the slab's last id
     for (int base = lo; base < hi; base += 128) {
