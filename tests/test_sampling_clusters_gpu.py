@@ -104,6 +104,54 @@ def test_every_draw_has_an_id(vocab):
         assert bool((behind <= 2e-5).all())
 
 
+@pytest.mark.parametrize("vocab", [5000, 20000, 70001])
+@pytest.mark.parametrize("listed", [1, 4095, 4096, 4097])
+def test_ids_at_the_lists_end(vocab, listed):
+    """`listed` ids of one weight stand in the bin that top-k and top-p fall into: the list takes 4,096, one more goes to the search by digits.  Equal
+    weights stand in the order of their ids, so the draw is known: of the k kept ones, or of those that weigh p times all (the others e^-60 of these)."""
+    from vllm_cpp_b200.csrc import ops
+    rng = np.random.default_rng(vocab + listed)
+    x = np.full((3, vocab), -50.0, dtype=np.float32)
+    for r in x:
+        r[rng.permutation(vocab)[:listed]] = 1.3
+    dev = lambda a, t: torch.from_numpy(np.asarray(a, dtype=t)).cuda()  # noqa: E731
+    k = min(10, listed)
+    for u in (0.0, 0.55, 1.0 - 2.0 ** -24):
+        out = torch.full((3,), -7, dtype=torch.int32, device="cuda")
+        ops.sample_filtered(dev(x, np.float32), dev([0.7, 0.7, 0.85], np.float32), dev([u] * 3, np.float32), dev([1.0, 0.5, 0.5], np.float32),
+                            dev([k, -1, k], np.int32), out)
+        kept = (k, (listed + 1) // 2, (k + 1) // 2)
+        assert out.tolist() == [int(np.flatnonzero(r > 0)[min(int(u * n), n - 1)]) for r, n in zip(x, kept)], (u, kept)
+
+
+@pytest.mark.parametrize("vocab", [300, 5000, 20000, 152064])
+def test_rows_that_are_no_numbers(vocab):
+    """Infinities and what is no number: a row gives an id of the vocabulary; the one +infinity is taken, -infinity and what is no number are not where
+    another id has weight."""
+    from vllm_cpp_b200.csrc import ops
+    x = np.random.default_rng(vocab).standard_normal((7, vocab)).astype(np.float32)
+    x[0] = np.nan
+    x[1] = -np.inf
+    x[2, vocab // 3] = np.inf
+    x[3, 1::2] = np.nan
+    x[4, ::2] = -np.inf
+    x[5] = np.finfo(np.float32).min
+    x[6, [1, vocab - 2]] = np.inf
+    dev = lambda a, t: torch.from_numpy(np.asarray(a, dtype=t)).cuda()  # noqa: E731
+    logits, u = dev(x, np.float32), dev([0.37] * 7, np.float32)
+    for temp in (1.0, 0.6):
+        for p, k in ((0.9, -1), (1.0, 40), (0.8, 7), (1.0 - 2.0 ** -24, vocab - 1)):
+            out = torch.full((7,), -7, dtype=torch.int32, device="cuda")
+            ops.sample_all(logits, dev([temp] * 7, np.float32), u, dev([p] * 7, np.float32), dev([k] * 7, np.int32), out)
+            got = out.tolist()
+            assert all(0 <= g < vocab for g in got), (temp, p, k, got)
+            assert got[2] == vocab // 3 and got[3] % 2 == 0 and got[4] % 2 == 1 and got[6] in (1, vocab - 2), (temp, p, k, got)
+        ops.sample(logits, dev([temp] * 7, np.float32), u, out.fill_(-7))
+        assert all(0 <= g < vocab for g in out.tolist())
+        ops.sample(logits, dev([0.0] * 7, np.float32), u, out.fill_(-7))
+        assert all(0 <= g < vocab for g in out.tolist()) and out.tolist()[2] == vocab // 3 and out.tolist()[6] == 1
+
+
 @pytest.mark.parametrize("vocab", [997, 70001])
 def test_all_rows_in_one_launch(vocab):
     """Greedy, plain and filtered rows side by side: what the two launches leave."""

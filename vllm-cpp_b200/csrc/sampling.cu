@@ -566,15 +566,16 @@ sample_filtered_kernel(const float* __restrict__ logits, int ld, int vocab, cons
     const bool vec = ((((uintptr_t)l) | ((uintptr_t)e)) & 15) == 0;
     FiltRow logit_row{l, first, last, ctas, vec, &sh}, weight_row{e, first, last, ctas, vec, &sh};
     float mx = -INFINITY;
-    logit_row.for_each([&](float v, int) { mx = fmaxf(mx, scaled ? v * inv_t : v); });
+    logit_row.for_each([&](float v, int) { mx = fmaxf(mx, scaled ? __fmul_rn(v, inv_t) : v); });
     mx = block_max(mx, red);
     if (threadIdx.x == 0) sh.cta_max = mx;
     weight_row.clear();
     cluster.sync();
     for (int c = 0; c < ctas; ++c) mx = fmaxf(mx, *cluster.map_shared_rank(&sh.cta_max, c));
     // (The largest has weight 1 even where the difference of two infinities would be no number; what is no number has no weight.)
+    // The product is rounded on its own wherever this is inlined: the ids counted and the ids gathered have the same weights.
     auto weight = [&](float v) {
-        const float x = scaled ? v * inv_t : v;
+        const float x = scaled ? __fmul_rn(v, inv_t) : v;
         const float w = x == mx ? 1.0f : expf(x - mx);
         return w <= 1.0f ? w : 0.0f;
     };
@@ -609,11 +610,12 @@ sample_filtered_kernel(const float* __restrict__ logits, int ld, int vocab, cons
         logit_row.for_each([&](float v, int id) {
             const float w = weight(v);
             if (__float_as_uint(w) < least) return;
-            list[atomicAdd(listed, 1)] = filt_key(w, id);
+            const int at = atomicAdd(listed, 1);
+            if (at < FILT_LIST) list[at] = filt_key(w, id);
         });
         cluster.sync();
         if (rank != 0) return;
-        const int id = filt_draw(sh, sh.listed, vocab, k, p, uniform[row], total);
+        const int id = filt_draw(sh, min(sh.listed, FILT_LIST), vocab, k, p, uniform[row], total);
         if (threadIdx.x == 0) out[row] = id;
         return;
     }
