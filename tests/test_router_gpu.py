@@ -42,3 +42,32 @@ def test_combine(n, width, top, dtype):
         want = (rows * (w.double()[..., None] if w is not None else 1.0)).sum(1) + (more.double() if more is not None else 0.0)
         # top + 1 float32 additions of numbers up to 5, and the stored type's rounding
         assert bool(((out.double() - want).abs() <= 1e-5 * (1 + want.abs()) + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)).all())
+
+
+@pytest.mark.parametrize("score", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("groups,keep", [(1, 1), (4, 2)])
+def test_choice_where_scores_are_no_numbers(score, groups, keep):
+    """Rows whose logits are infinite or no numbers, and corrections of -infinity: every choice is another output, the lowest ones among those without a
+    score, and a row's neighbours are not touched."""
+    from vllm_cpp_b200.csrc import ops
+    n, width, outs, top = 9, 64, 40, 6
+    gen = torch.Generator(device="cuda").manual_seed(groups)
+    h, w = torch.randn(n, width, device="cuda", generator=gen), torch.randn(outs, width, device="cuda", generator=gen)
+    plain = h.clone()
+    h[1], h[3, 5], h[5, 7], h[7, 0] = float("nan"), float("nan"), float("inf"), -float("inf")
+    never = torch.zeros(outs, device="cuda")
+    never[4:] = -float("inf")                                             # four outputs are left for six choices
+    for correction in (None, never):
+        got = []
+        for rows in (h, plain):
+            ids, weights = torch.full((n, top), -7, dtype=torch.int32, device="cuda"), torch.empty(n, top, device="cuda")
+            ops.moe_router(rows, w, correction, ids, weights, torch.empty(n, outs, device="cuda"), score=score, groups=groups, keep_groups=keep, group_top=2)
+            assert int(ids.min()) >= 0 and int(ids.max()) < outs
+            assert all(len(set(r)) == top for r in ids.tolist())
+            got.append((ids, weights))
+        clean = [0, 2, 4, 6, 8]
+        assert torch.equal(got[0][0][clean], got[1][0][clean]) and torch.equal(got[0][1][clean], got[1][1][clean])
+        if groups == 1:
+            assert got[0][0][1].tolist() == list(range(top))              # nothing has a score
+        if correction is not None and groups == 1:
+            assert all(set(range(4)) <= set(r) for r in got[1][0].tolist())

@@ -204,7 +204,7 @@ moe_router_select_kernel(const float* __restrict__ logits, const float* __restri
     const int t = blockIdx.x * 4 + warp;
     if (t >= n_tokens) return;
     float* score = sm + (size_t)warp * (2 * n_out + rule.n_groups);      // [n_out] scores
-    float* choice = score + n_out;                     // [n_out] score + correction; -inf once taken or shut out
+    float* choice = score + n_out;                     // [n_out] score + correction (-inf where that is no number); no number once taken or shut out
     float* gscore = choice + n_out;                    // [n_groups]
     const float* zr = logits + (size_t)t * n_out;
     auto z = [&](int e) { return logit_bias ? zr[e] + logit_bias[e] : zr[e]; };      // the router's bias joins the logits themselves (float)
@@ -219,7 +219,10 @@ moe_router_select_kernel(const float* __restrict__ logits, const float* __restri
     } else {
         for (int e = lane; e < n_out; e += 32) score[e] = 1.0f / (1.0f + expf(-z(e)));
     }
-    for (int e = lane; e < n_out; e += 32) choice[e] = score[e] + (correction ? correction[e] : 0.0f);
+    for (int e = lane; e < n_out; e += 32) {
+        const float v = score[e] + (correction ? correction[e] : 0.0f);
+        choice[e] = v == v ? v : -INFINITY;
+    }
     __syncwarp();
     if (rule.n_groups > 1 && rule.keep_groups < rule.n_groups) {
         const int per = n_out / rule.n_groups;
@@ -257,24 +260,26 @@ moe_router_select_kernel(const float* __restrict__ logits, const float* __restri
             __syncwarp();
         }
         for (int e = lane; e < n_out; e += 32)
-            if (gscore[e / per] != INFINITY) choice[e] = -INFINITY;
+            if (gscore[e / per] != INFINITY) choice[e] = NAN;
         __syncwarp();
     }
     for (int k = 0; k < top; ++k) {
         float best = -INFINITY;
         int at = 0x7fffffff;
-        for (int e = lane; e < n_out; e += 32)
-            if (choice[e] > best) { best = choice[e]; at = e; }        // the lowest index among equals of a lane
+        for (int e = lane; e < n_out; e += 32) {
+            const float v = choice[e];
+            if (v > best || (v == -INFINITY && at == 0x7fffffff)) { best = v; at = e; }        // the lowest index among equals of a lane
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const float ob = __shfl_xor_sync(0xffffffffu, best, o);
             const int oa = __shfl_xor_sync(0xffffffffu, at, o);
             if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; }
         }
-        if (lane == 0) {
+        if (lane == 0) {                               // `at` is an output: the kept groups hold `top` and more (checked at the launch)
             ids[(size_t)t * top + k] = at;
             wts[(size_t)t * top + k] = score[at];
-            choice[at] = -INFINITY;
+            choice[at] = NAN;
         }
         __syncwarp();
     }
