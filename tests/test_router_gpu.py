@@ -26,6 +26,21 @@ def test_logits_and_choice(n, width, outs, dtype):
     assert bool(((weights.double() - torch.sigmoid(logits.double()).gather(1, ids.long())).abs() <= 1e-6).all())
 
 
+@pytest.mark.parametrize("n,width", [(3, 1028), (8, 4), (5, 3076), (65, 1028), (3, 1030)])
+def test_logits_of_infinite_activations(n, width):
+    """An infinite activation gives infinite logits, of its weight's sign; other tokens' logits do not see it."""
+    from vllm_cpp_b200.csrc import ops
+    outs = 12
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    h, w = torch.randn(n, width, device="cuda", generator=gen), torch.randn(outs, width, device="cuda", generator=gen)
+    h[0, 1], h[2, width - 2] = float("inf"), -float("inf")
+    ids, weights, logits = torch.empty(n, 2, dtype=torch.int32, device="cuda"), torch.empty(n, 2, device="cuda"), torch.empty(n, outs, device="cuda")
+    ops.moe_router(h, w, None, ids, weights, logits, score="sigmoid")
+    assert torch.equal(logits[0], torch.sign(w[:, 1]) * float("inf")) and torch.equal(logits[2], -torch.sign(w[:, width - 2]) * float("inf"))
+    rest = [t for t in range(n) if t not in (0, 2)]
+    assert bool(((logits[rest].double() - h[rest].double() @ w.double().T).abs() <= 1e-5 * width ** 0.5).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,width,top", [(1, 4, 1), (5, 1028, 3), (7, 1024, 4), (9, 132, 5), (3, 4096, 9), (6, 130, 3)])
 def test_combine(n, width, top, dtype):

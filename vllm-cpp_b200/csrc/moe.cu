@@ -118,7 +118,8 @@ moe_router_few_kernel(const T* __restrict__ h, long long ldh, const float* __res
         for (int t = 0; t < RT_FEW_TOK; ++t) {
             const T* row = h + (size_t)min(t0 + t, n_tokens - 1) * ldh;        // rows beyond the last repeat it; they are not stored
             x[t] = router_piece<T>(row + k);
-            y[t] = router_piece<T>(row + (second ? k + 1024 : k));
+            // (not the first piece again: an infinite activation times the zeros of `b` would be no number)
+            y[t] = second ? router_piece<T>(row + k + 1024) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
 #pragma unroll
         for (int t = 0; t < RT_FEW_TOK; ++t) acc[t] = dot4(y[t], b, dot4(x[t], a, acc[t]));
