@@ -1,4 +1,4 @@
-"""Router logits of few tokens (a CTA per output), of many (two, five and eight outputs a warp) and of rows that 4-element pieces do not cover, and the
+"""Router logits of few tokens (a warp per output and one or two tokens), of many (two, three and five outputs a warp) and of rows that 4-element pieces do not cover, and the
 choices' rows joined four elements at a time and one at a time; against 64 bits."""
 import pytest
 import torch
@@ -24,6 +24,27 @@ def test_logits_and_choice(n, width, outs, dtype):
     assert bool(((logits.double() - want).abs() <= 1e-5).all())
     assert torch.equal(ids.long(), logits.topk(top, dim=1).indices)
     assert bool(((weights.double() - torch.sigmoid(logits.double()).gather(1, ids.long())).abs() <= 1e-6).all())
+
+
+# one kernel or another by the number of logits: 1 and 8 tokens a warp each, then two tokens a warp, then many
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("outs,width", [(3, 4), (16, 132), (33, 1028), (64, 4096), (130, 260), (17, 1030)])
+def test_logits_do_not_depend_on_the_step(outs, width, dtype):
+    """A token's logits are the same bits in whichever step it stands, so a near tie is decided alike."""
+    from vllm_cpp_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(outs)
+    h, w = torch.randn(700, width, device="cuda", generator=gen).to(dtype), torch.randn(outs, width, device="cuda", generator=gen)
+
+    def logits(rows):
+        n, z = rows.shape[0], torch.empty(rows.shape[0], outs, device="cuda")
+        ops.moe_router(rows, w, None, torch.empty(n, 1, dtype=torch.int32, device="cuda"), torch.empty(n, 1, device="cuda"), z, score="sigmoid")
+        return z
+    whole = logits(h)
+    for n in (1, 8, 64, 65, 76, 150, 301):
+        assert torch.equal(logits(h[:n]), whole[:n]), n
+    odd = torch.empty(5, width + 1, dtype=dtype, device="cuda")[:, :width]      # rows that pieces do not cover: the third kernel
+    if width % 4 == 0:
+        assert torch.equal(logits(odd.copy_(h[:5])), whole[:5])
 
 
 @pytest.mark.parametrize("n,width", [(3, 1028), (8, 4), (5, 3076), (65, 1028), (3, 1030)])

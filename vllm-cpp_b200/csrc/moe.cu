@@ -24,12 +24,16 @@
 #include <cuda.h>
 
 // ------------------------------------------------------------------------------------------- router
-// Logits, then selection.  Logits: where 4-element pieces cover the rows, two kernels.  Few tokens: a CTA per router output and eight
-// tokens, its 256 threads split the row, so that a row of 4,096 is four independent loads of the matrix and 32 of the tokens a thread
-// (8 tokens, 33 outputs of 4,096: 6.5 us).  Many: eight tokens a CTA, a warp four to eight outputs, so that a
-// token's piece is read for several outputs and a matrix's piece for eight tokens (2,048 tokens: 36 us; 16 calls of 8 tokens and two of
-// 2,048 took 398 us with a warp per output and four tokens in shared memory, now 176).  Else a CTA takes RT_TOK tokens and eight router outputs, a warp per output: the tokens' rows pass
-// through shared memory in slabs (as float).  Selection: a warp per token does the softmax over all outputs, adds the correction and
+// Logits, then selection.  A logit is one sum in one order whatever the step's other tokens are, so a token's experts do not depend
+// on them: lane l of a warp adds up the row's pieces of four elements l, l + 32, .. one after another, then the lanes are joined.  Three
+// kernels with that order, taken by speed alone where 4-element pieces cover the rows:
+//   rows   a warp per output and one or two tokens, eight pieces of both rows in flight a lane: bound by those round trips to L2 (8 tokens, 33
+//          outputs of 4,096: 4.3 us, 12.2 with the last of the three; 128 tokens, 64 outputs: 11.2 and 16.0)
+//   many   eight tokens and two, three or five outputs a warp, so that a token's piece is read for several outputs and a matrix's piece
+//          for eight tokens: bound by the FMAs' operands (2,048 tokens, 33 outputs of 4,096: 35 us, 87 with the kernel below)
+//   else   a CTA takes RT_TOK tokens and eight router outputs, a warp per output: the tokens' rows pass through shared memory in
+//          slabs (as float); short rows, and those that pieces do not cover.
+// Selection: a warp per token does the softmax over all outputs, adds the correction and
 // picks the `top` largest (the lower index wins among equals); the plain scores of the chosen are the weights.
 #define RT_TOK 4
 #define RT_SLAB 2048
@@ -99,41 +103,43 @@ template <> __device__ __forceinline__ float4 router_piece<__nv_bfloat16>(const 
 }
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c)))); }
 
-constexpr int RT_FEW_TOK = 8;
-template <typename T>
+template <typename T, int TOK>
 __global__ void __launch_bounds__(256)
-moe_router_few_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr, float* __restrict__ logits, int n_tokens, int width, int n_out) {
-    __shared__ float sums[8][RT_FEW_TOK];
-    const int t0 = blockIdx.x * RT_FEW_TOK, e = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float* w = wr + (size_t)e * width;
-    float acc[RT_FEW_TOK];
-#pragma unroll
-    for (int t = 0; t < RT_FEW_TOK; ++t) acc[t] = 0.0f;
+moe_router_rows_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr, float* __restrict__ logits, int n_tokens, int width, int n_out) {
+    constexpr int AHEAD = 8;
+    const int lane = threadIdx.x & 31, groups = (n_tokens + TOK - 1) / TOK;
+    const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     pdl_start();
-    for (int k = threadIdx.x * 4; k < width; k += 2048) {
-        const bool second = k + 1024 < width;
-        const float4 a = router_piece<float>(w + k), b = second ? router_piece<float>(w + k + 1024) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float4 x[RT_FEW_TOK], y[RT_FEW_TOK];
+    if (item >= (long long)groups * n_out) return;
+    const int e = (int)(item / groups), t0 = (int)(item % groups) * TOK;
+    const float* w = wr + (size_t)e * width;
+    const T* row[TOK];
+    float acc[TOK];
 #pragma unroll
-        for (int t = 0; t < RT_FEW_TOK; ++t) {
-            const T* row = h + (size_t)min(t0 + t, n_tokens - 1) * ldh;        // rows beyond the last repeat it; they are not stored
-            x[t] = router_piece<T>(row + k);
-            // (not the first piece again: an infinite activation times the zeros of `b` would be no number)
-            y[t] = second ? router_piece<T>(row + k + 1024) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int t = 0; t < TOK; ++t) {
+        row[t] = h + (size_t)min(t0 + t, n_tokens - 1) * ldh;              // rows beyond the last repeat it; they are not stored
+        acc[t] = 0.0f;
+    }
+    for (int k = lane * 4; k < width; k += 128 * AHEAD) {
+        float4 a[AHEAD], x[AHEAD][TOK];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            if (k + 128 * u >= width) continue;
+            a[u] = router_piece<float>(w + k + 128 * u);
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) x[u][t] = router_piece<T>(row[t] + k + 128 * u);
         }
 #pragma unroll
-        for (int t = 0; t < RT_FEW_TOK; ++t) acc[t] = dot4(y[t], b, dot4(x[t], a, acc[t]));
+        for (int u = 0; u < AHEAD; ++u) {
+            if (k + 128 * u >= width) continue;
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) acc[t] = dot4(x[u][t], a[u], acc[t]);
+        }
     }
 #pragma unroll
-    for (int t = 0; t < RT_FEW_TOK; ++t) {
+    for (int t = 0; t < TOK; ++t) {
         const float v = warp_sum(acc[t]);
-        if (lane == 0) sums[warp][t] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < RT_FEW_TOK && t0 + (int)threadIdx.x < n_tokens) {
-        float v = 0.0f;
-        for (int q = 0; q < 8; ++q) v += sums[q][threadIdx.x];
-        logits[(size_t)(t0 + threadIdx.x) * n_out + e] = v;
+        if (lane == 0 && t0 + t < n_tokens) logits[(size_t)(t0 + t) * n_out + e] = v;
     }
 }
 
@@ -173,16 +179,26 @@ moe_router_many_kernel(const T* __restrict__ h, long long ldh, const float* __re
 template <typename T>
 static void launch_router_logits(const T* h, long long ldh, const float* wr, float* logits, int n_tokens, int width, int n_out, cudaStream_t s) {
     if ((width & 3) == 0 && (ldh & 3) == 0 && (((uintptr_t)wr) & 15) == 0 && (((uintptr_t)h) & (4 * sizeof(T) - 1)) == 0) {
-        // few: as long as the CTAs per output leave the device room
-        if (n_tokens <= 64 && n_out <= 65535) {
-            vcb_launch(moe_router_few_kernel<T>, dim3((n_tokens + RT_FEW_TOK - 1) / RT_FEW_TOK, n_out), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
-            return;
-        }
-        const int blocks = (n_tokens + 7) / 8;
-        if (n_out <= 16) vcb_launch(moe_router_many_kernel<T, 2>, dim3(blocks, (n_out + 15) / 16), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
-        else if (n_out <= 40) vcb_launch(moe_router_many_kernel<T, 5>, dim3(blocks, (n_out + 39) / 40), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
-        else vcb_launch(moe_router_many_kernel<T, 8>, dim3(blocks, (n_out + 63) / 64), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
-        return;
+        // By the number of logits, measured over 1 to 2,048 tokens, 3 to 256 outputs and widths of 64 to 7,168: a warp each up to 2,500; up to 10,000
+        // a warp for two tokens (64 tokens, 64 outputs of 4,096: 6.6 us, many 18.4), but not for short rows, whose many warps wait for little
+        // each (64 tokens, 130 outputs of 64: 4.0 us, the kernel below 2.7); above, five outputs a warp in float32 (2,048 x 64 of 4,096: 46 us,
+        // three 58), three in bfloat16 (58 and 63 us: its conversions) and where 24 outputs or fewer leave warps of five idle, two for short rows.
+        const long long count = (long long)n_tokens * n_out;
+        const auto rows = [&](auto kernel, int tok) {
+            const long long items = (long long)((n_tokens + tok - 1) / tok) * n_out;
+            vcb_launch(kernel, (unsigned)((items + 7) / 8), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
+        };
+        const auto many = [&](auto kernel, int outs) {
+            vcb_launch(kernel, dim3((n_tokens + 7) / 8, (n_out + 8 * outs - 1) / (8 * outs)), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
+        };
+        bool taken = true;
+        if (count <= 2500) rows(moe_router_rows_kernel<T, 1>, 1);
+        else if (count <= 10000 && width >= 512) rows(moe_router_rows_kernel<T, 2>, 2);
+        else if (count <= 10000) taken = false;
+        else if (width < 512) many(moe_router_many_kernel<T, 2>, 2);
+        else if (sizeof(T) == 4 && count > 20000 && n_out > 24) many(moe_router_many_kernel<T, 5>, 5);
+        else many(moe_router_many_kernel<T, 3>, 3);
+        if (taken) return;
     }
     vcb_launch(moe_router_logits_kernel<T>, dim3((n_tokens + RT_TOK - 1) / RT_TOK, (n_out + 7) / 8), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
 }
