@@ -48,6 +48,29 @@ def test_gated_delta_walk(reqs, H, G, dk, dv):
     assert bool((state.double()[rest] == S0[rest]).all())
 
 
+# of 148 SMs: one column a thread alone, two or four beside others; 8, 16 and 32 lanes a column, and keys whose last lanes are padding
+@pytest.mark.parametrize("H,G,dk,dv", [(8, 4, 64, 40), (8, 4, 50, 24), (16, 8, 128, 64), (8, 8, 130, 36), (6, 3, 300, 64), (8, 4, 30, 40)])
+def test_walk_does_not_depend_on_the_step(H, G, dk, dv):
+    """A request's outputs and state are the same bits alone and beside 1, 3, 11 and 80 others."""
+    from vllm_cpp_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(dk)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    lens = [23] + [17, 9, 23, 8, 12] * 16
+    n = sum(lens)
+    q, k, v = rnd(n, G * dk), rnd(n, G * dk), rnd(n, H * dv)
+    beta, dec, a_log, dt, first = rnd(n, H), rnd(n, H * dk), 0.1 * rnd(H), rnd(H * dk), rnd(len(lens), H, dk, dv)
+    seen = None
+    for reqs in (1, 2, 4, 12, len(lens)):
+        m = sum(lens[:reqs])
+        start = torch.tensor([sum(lens[:r]) for r in range(reqs + 1)], dtype=torch.int32, device="cuda")
+        state, out = first[:reqs].clone(), torch.full((m, H * dv), 9.0, device="cuda")
+        ops.gated_delta_scan(q[:m], k[:m], v[:m], beta[:m], dec[:m], a_log, dt, state, out, start, torch.arange(reqs, dtype=torch.int32, device="cuda"),
+                             reqs, num_heads=H, num_qk_heads=G, q_scale=dk ** -0.5, unit_eps=1e-6, max_q_len=23)
+        got = (out[:23].clone(), state[0].clone())
+        assert seen is None or (torch.equal(seen[0], got[0]) and torch.equal(seen[1], got[1])), reqs
+        seen = seen or got
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,B,bs", [(33, 3, 8), (64, 2, 64), (65, 2, 72), (130, 1, 136), (100, 3, 20), (70, 2, 33)])
 def test_gates(dtype, n, B, bs):

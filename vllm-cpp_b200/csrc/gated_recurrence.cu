@@ -768,9 +768,11 @@ __device__ __forceinline__ void walk_copy(float* smem, const float* gmem, int by
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(gmem) : "memory");
 }
 
-// s[0 .. N) summed over the lanes whose numbers differ in the bits from BIT down; lane l ends with sum l / (2 BIT / N) in s[0].
+// s[0 .. N) summed over P lanes, neighbours first: the pairs, then the pairs' sums and so on, the order of a butterfly from bit 0 up, so that a
+// column's sums are the same bits here and in the walk of one column a thread.  While a lane holds several sums an exchange halves them, so
+// lane `part` ends with the sum whose number is its low bits reversed (walk_reversed), in s[0].
 template <int N>
-__device__ __forceinline__ void walk_halve(float* s, int part, int bit) {
+__device__ __forceinline__ void walk_halve(float* s, int part, int bit, int P) {
     if constexpr (N > 1) {
         const bool upper = (part & bit) != 0;
 #pragma unroll
@@ -778,10 +780,14 @@ __device__ __forceinline__ void walk_halve(float* s, int part, int bit) {
             const float keep = upper ? s[i + N / 2] : s[i], give = upper ? s[i] : s[i + N / 2];
             s[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
         }
-        walk_halve<N / 2>(s, part, bit >> 1);
+        walk_halve<N / 2>(s, part, bit << 1, P);
     } else {
-        for (; bit >= 1; bit >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+        for (; bit < P; bit <<= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
     }
+}
+// the low bits of x, as many as N = 2, 4 or 8 sums have, in reverse
+template <int N> __host__ __device__ constexpr int walk_reversed(int x) {
+    return N == 8 ? ((x & 1) << 2) | (x & 2) | ((x >> 2) & 1) : N == 4 ? ((x & 1) << 1) | ((x >> 1) & 1) : x & 1;
 }
 
 template <int DKP, int COLS>
@@ -853,7 +859,7 @@ delta_walk_kernel(DeltaArgs a, const float* __restrict__ work, long long ldw, in
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (row0 < row1) fetch(row0, 0);
-    const int rep = P / (2 * COLS);           // lanes that end with the same sum; P is at least 8
+    const int held = walk_reversed<2 * COLS>(part);       // the sum this lane ends with; P is at least 8
     const int lane0 = (tid & 31) - part;           // the first lane of this column group
     int b = 0;
     for (int c0 = row0; c0 < row1; c0 += TC, b ^= 1) {
@@ -905,18 +911,17 @@ delta_walk_kernel(DeltaArgs a, const float* __restrict__ work, long long ldw, in
                 s[c] = sum2f(p0) + sum2f(p1);
                 s[COLS + c] = sum2f(r0) + sum2f(r1);
             }
-            walk_halve<2 * COLS>(s, part, P >> 1);
+            walk_halve<2 * COLS>(s, part, 1, P);
             float mine_u = 0.0f;                   // u of the column whose r this lane ends with
-            const int held = part / rep;
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
-                const float u = w.beta * (w.v[c] - __shfl_sync(0xffffffffu, s[0], lane0 + c * rep));
+                const float u = w.beta * (w.v[c] - __shfl_sync(0xffffffffu, s[0], lane0 + walk_reversed<2 * COLS>(c)));
                 const f32x2 uu = pack2f(u, u);
 #pragma unroll
                 for (int i = 0; i < DKP / 2; ++i) S[c][i] = fma2f(w.k[i], uu, S[c][i]);
                 if (held == COLS + c) mine_u = u;
             }
-            if (held >= COLS && part % rep == 0) os[tt * DVT + cl + held - COLS] = fmaf(w.qk, mine_u, s[0]);
+            if (held >= COLS && part < 2 * COLS) os[tt * DVT + cl + held - COLS] = fmaf(w.qk, mine_u, s[0]);
         };
         Rows even, odd;
         read(even, 0);
