@@ -6,14 +6,16 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# requests, heads, qk heads: with 148 SMs 4 * requests * heads * (value channels / columns a CTA) is from 1,480 on for four columns, else two, else one
-@pytest.mark.parametrize("reqs,H,G,dk,dv", [(33, 16, 8, 30, 40), (33, 16, 16, 128, 70), (33, 12, 4, 130, 36), (12, 16, 4, 30, 40), (40, 10, 5, 64, 32),
-                                            (3, 6, 3, 128, 40), (2, 4, 1, 36, 20), (2, 3, 3, 300, 70)])
+# requests, heads, qk heads: with 148 SMs 4 * (tokens / 21) * heads * (value channels / columns a CTA) is from 1,480 on for four columns, from 1,184 on for two, else
+# one, as for keys of up to 32 channels; two as well for keys beyond 256, and (the last) for a prompt beside many single tokens
+@pytest.mark.parametrize("reqs,H,G,dk,dv", [(33, 16, 8, 30, 40), (33, 16, 16, 128, 70), (33, 12, 4, 130, 36), (12, 16, 4, 30, 40), (40, 10, 5, 64, 32), (12, 8, 8, 64, 70),
+                                            (3, 6, 3, 128, 40), (2, 4, 1, 36, 20), (2, 3, 3, 300, 70), (120, 8, 8, 300, 40), (-7, 8, 4, 40, 36)])
 def test_gated_delta_walk(reqs, H, G, dk, dv):
     from vllm_cpp_b200.csrc import ops
     gen = torch.Generator(device="cuda").manual_seed(reqs + dk)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
-    lens = [1 + (7 * r) % 19 for r in range(reqs)]
+    lens = [1 + (7 * r) % 19 if reqs > 0 else 1 for r in range(abs(reqs))]
+    reqs = len(lens)
     lens[0] = 21
     n = sum(lens)
     start = [0]

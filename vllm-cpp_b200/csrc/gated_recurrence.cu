@@ -1115,7 +1115,7 @@ static int launch_walk(DeltaArgs b, int n_reqs, const float* work, long long ldw
 }
 
 template <typename T>
-static int launch_delta_portions(const DeltaArgs& a, int n_reqs, int n_tokens, float* work, cudaStream_t s) {
+static int launch_delta_portions(const DeltaArgs& a, int n_reqs, int n_tokens, int max_q_len, float* work, cudaStream_t s) {
     // 8 rows of a column per thread where the key channels fill 16 lanes (keys of 128), fewer lanes for shorter keys, 16 rows for longer
     // ones; CTAs of four warps, so that a head's columns spread over many SMs.
     const int dkp = a.dk > 256 ? 16 : 8;
@@ -1130,16 +1130,23 @@ static int launch_delta_portions(const DeltaArgs& a, int n_reqs, int n_tokens, f
     const long long items = (long long)n_tokens * a.H;
     vcb_launch(delta_prepare_kernel<T>, dim3((unsigned)((items + 3) / 4)), 128, 0, s, a, work, ldw, n_tokens);
     if (int e = vcb_last_error()) return e;
-    // Columns a thread: four or two where the device still has two and a half warps a scheduler then (32 heads of 128 x 128, us with
-    // one / two / four: 8 prompts of together 2,048 tokens 1,093 / 704 / 645, 3 of 700 1,129 / 792 / 606, 2 of together 1,024 682 / 448 /
-    // 540, 1 of 2,048 1,176 / 1,359 / 1,654).  They need at least eight lanes a column group (the eight sums of four columns then end in
-    // lanes of their own), which keys below 64 channels leave partly idle.
-    const int lanes = P < 8 ? 8 : P;
-    const auto warps = [&](int cols) { const int w = 128 / lanes * cols; return 4LL * n_reqs * a.H * ((a.dv + w - 1) / w); };
-    const long long enough = 10LL * vcb_sm_count();
-    const int cols = warps(4) >= enough ? 4 : warps(2) >= enough ? 2 : 1;
-    if (cols == 4) return dkp == 8 ? launch_walk<8, 4>(a, n_reqs, work, ldw, lanes, s) : launch_walk<16, 4>(a, n_reqs, work, ldw, lanes, s);
-    if (cols == 2) return dkp == 8 ? launch_walk<8, 2>(a, n_reqs, work, ldw, lanes, s) : launch_walk<16, 2>(a, n_reqs, work, ldw, lanes, s);
+    // Columns a thread: more of them where the device still has warps enough while the longest portion is walked.  Requests count by their
+    // share of it, n_tokens / max_q_len: those of a single token beside a prompt are done after a token and leave it alone (32 heads of
+    // 128 x 128, us with one / two / four columns: a prompt of 600 beside two single tokens 376 / 396 / 492; 8 prompts of together 2,048 tokens
+    // 1,093 / 704 / 645, 3 of 700 1,129 / 792 / 606, 2 of together 1,024 682 / 448 / 540, 1 of 2,048 1,176 / 1,359 / 1,654).  Four from two and
+    // a half warps a scheduler on, two from two on; and two where single tokens are many for the prompt's length, because then their states' way in and
+    // out decides, which wider rows shorten (500 and 63 single tokens 700 / 520 / 538).  Keys beyond 256 channels, whose lanes are a whole
+    // warp a column, take two at least (16 heads of 512 x 64, 600 tokens: 557 / 425), and keys of up to 32 channels one: the sums of
+    // several columns end in at least eight lanes, of which theirs leave half idle (64 heads of 16 x 128, 8 prompts of 256: 274 / 556 / 512).
+    const auto warps = [&](int cols) { const int w = 128 / P * cols; return 4LL * a.H * ((a.dv + w - 1) / w); };      // of a request
+    const long long sms = vcb_sm_count(), longest = max_q_len > 0 ? max_q_len : 1;
+    int cols = 1;
+    if (P >= 8) {
+        if (warps(4) * n_tokens >= 10 * sms * longest) cols = 4;
+        else if (warps(2) * n_tokens >= 8 * sms * longest || warps(2) * n_reqs >= 16 * longest || P == 32) cols = 2;
+    }
+    if (cols == 4) return dkp == 8 ? launch_walk<8, 4>(a, n_reqs, work, ldw, P, s) : launch_walk<16, 4>(a, n_reqs, work, ldw, P, s);
+    if (cols == 2) return dkp == 8 ? launch_walk<8, 2>(a, n_reqs, work, ldw, P, s) : launch_walk<16, 2>(a, n_reqs, work, ldw, P, s);
     DeltaArgs b = a;
     b.chunk = chunk;
     const dim3 grid(n_reqs, a.H, (a.dv + dvt - 1) / dvt);
@@ -1175,7 +1182,7 @@ VCB_EXPORT int vcb_gated_delta_scan(const float* q, const float* k, const float*
                                     const void* beta_pre, long long ldb, const void* decay_pre, long long lda,
                                     const float* a_log, const float* dt_bias, float* state, float* out, long long ldo,
                                     const int* q_start, const int* state_slots, int n_reqs, int H, int G, int dk, int dv,
-                                    float q_scale, float unit_eps, int dtype, float* work, int n_tokens, void* stream) {
+                                    float q_scale, float unit_eps, int dtype, float* work, int n_tokens, int max_q_len, void* stream) {
     if (n_reqs <= 0) return 0;
     if (!q || !k || !v || !beta_pre || !decay_pre || !a_log || !dt_bias || !state || !out || H <= 0 || G <= 0 || H % G ||
         dk <= 0 || dv <= 0 || H > 65535 || (dv + 7) / 8 > 65535)
@@ -1184,8 +1191,8 @@ VCB_EXPORT int vcb_gated_delta_scan(const float* q, const float* k, const float*
                 H, G, dk, dv, q_scale, unit_eps, 0};
     cudaStream_t s = (cudaStream_t)stream;
     if (work && n_tokens > 0) {                   // a step with portions: inputs prepared for all tokens at once, then the walk
-        if (dtype == VCB_F32) return launch_delta_portions<float>(a, n_reqs, n_tokens, work, s);
-        if (dtype == VCB_BF16) return launch_delta_portions<__nv_bfloat16>(a, n_reqs, n_tokens, work, s);
+        if (dtype == VCB_F32) return launch_delta_portions<float>(a, n_reqs, n_tokens, max_q_len, work, s);
+        if (dtype == VCB_BF16) return launch_delta_portions<__nv_bfloat16>(a, n_reqs, n_tokens, max_q_len, work, s);
         return VCB_ERR_BAD_ARG;
     }
     if (dtype == VCB_F32) return launch_delta<float>(a, n_reqs, s);

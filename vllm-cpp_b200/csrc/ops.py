@@ -102,7 +102,7 @@ _SIGNATURES = {
     "vcb_pair_norm": [_P, _P, _P, _P, _F, _F, _F, _P, _P, _P, _P, _I, _I, _F, _F, _I, _P],
     "vcb_gate_blocks": [_P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _I, _I, _I, _F, _I, _P],
     "vcb_linear_recurrence": [_P, _P, _L, _P, _L, _P, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _P],
-    "vcb_gated_delta_scan": [_P, _P, _P, _L, _L, _L, _P, _L, _P, _L, _P, _P, _P, _P, _L, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _P, _I, _P],
+    "vcb_gated_delta_scan": [_P, _P, _P, _L, _L, _L, _P, _L, _P, _L, _P, _P, _P, _P, _L, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _P, _I, _I, _P],
     "vcb_add_tanh_norm": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _F, _F, _I, _P],
     "vcb_act_rows": [_P, _P, _L, _I, _I, _P],
     "vcb_state_dual": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _P, _L, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
@@ -1511,7 +1511,7 @@ def gated_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_pre
                                       state.data_ptr(), out.data_ptr(), out.stride(0), _dev(q_start, "q_start", torch.int32),
                                       _dev(state_slots, "state_slots", torch.int32), n_reqs, H, G, dk, dv, float(q_scale),
                                       float(unit_eps), dtype_code(beta_pre.dtype), work.data_ptr() if portions else None,
-                                      n if portions else 0, _stream()), "gated_delta_scan")
+                                      n if portions else 0, max_q_len, _stream()), "gated_delta_scan")
 
 
 # ------------------------------------------------- attention over a window of tokens and means of blocks before it
