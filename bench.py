@@ -1767,14 +1767,15 @@ def rufisun_kernels(z, peaks):
     E, top, ef = z["experts"], z["top"], z["expert_ff"]
     w1, w2 = rnd(E, ef, h, scale=0.02), rnd(E, 2 * ef, h, scale=0.02)
     for t in (8, 64, 2048):
-        tm, pairs = ops.moe_tile_rows(t, top, E), t * top
+        pairs, xs = t * top, rnd(t, h)
+        tm = ops.moe_tile_rows(t, top, E, tensor_cores=ops.moe_tensor_tiles(xs, h, ef))
         tiles = ops.moe_max_tiles(t, top, E, tm)
         ids = torch.stack([torch.randperm(E, device=dev)[:top] for _ in range(t)]).to(torch.int32).contiguous()
         ints = [torch.empty(n, dtype=torch.int32, device=dev) for n in (pairs, pairs, tiles, tiles, tiles, 4)]
         wts, rs = torch.rand(t, top, device=dev), torch.empty(pairs, device=dev)
         ops.moe_sort(ids, E, tm, *ints, wts, rs)
         st, _, te, t0, tr, meta = ints
-        xs, act = rnd(t, h), torch.empty(pairs, ef, dtype=bf, device=dev)
+        act = torch.empty(pairs, ef, dtype=bf, device=dev)
         used = int(torch.unique(ids).numel())
         size = (lambda n: dict(bytes_=used * n * h * 2)) if t <= 64 else (lambda n: dict(flops=2.0 * pairs * n * h))
         add(f"experts' first product + gelu of the weighted input, {E} of {ef}, top {top}, {t} tokens", "", lambda i: ops.moe_expert_gemm(

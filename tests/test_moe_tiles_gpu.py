@@ -67,3 +67,35 @@ def test_products(n, experts, top, N, K, mode):
         else:
             want = z
         assert bool(((got[at] - want).abs() <= tol).all()), (mode, e)
+
+
+@pytest.mark.parametrize("step,first", [(64, 0), (72, 8), (66, 0), (72, 1)])
+def test_rows_that_16_byte_copies_do_not_fit(step, first):
+    """Tokens' rows anywhere: those at other than 16-byte boundaries take the products that read single elements."""
+    from vllm_cpp_b200.csrc import ops
+    from vllm_cpp_b200.parts.base import Workspace
+    from vllm_cpp_b200.parts.moe import RoutedExperts
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    n, width, ff, experts, top = 300, 64, 72, 4, 2
+    part = RoutedExperts(width, ff, experts, 0, top, 1.5, torch.bfloat16, "cuda", correction=False)
+    params = {"router": rnd(experts, width)}
+    for e in range(experts):
+        params.update({f"e{e}.gate": (rnd(ff, width) / 8).bfloat16(), f"e{e}.up": (rnd(ff, width) / 8).bfloat16(), f"e{e}.down": (rnd(width, ff) / 8).bfloat16()})
+    part.load_params(params)
+    x = torch.empty(n * step + first, dtype=torch.bfloat16, device="cuda")[first:].view(n, step)[:, :width].copy_(rnd(n, width))
+    assert ops.moe_tensor_tiles(x, width, ff) == (step != 66 and first != 1)
+    out, z = torch.empty(n, width, dtype=torch.bfloat16, device="cuda"), x.double() @ params["router"].double().T
+    part.forward(x, out, None, Workspace("cuda"))
+    ops.check_status()
+    p = torch.softmax(z, 1)
+    best, ids = p.topk(top, dim=1)
+    want = torch.zeros(n, width, dtype=torch.float64, device="cuda")
+    for e in range(experts):
+        g, u = (x.double() @ params[f"e{e}.{m}"].double().T for m in ("gate", "up"))
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+        act = (g * torch.sigmoid(1.702 * g) * (u + 1.0)).bfloat16().double()
+        want += (act @ params[f"e{e}.down"].double().T) * (best * (ids == e)).sum(1, keepdim=True)
+    clear = (p.topk(top + 1, dim=1).values.diff(dim=1)[:, -1].abs() > 1e-4)
+    # the activation's rounding, which falls the other way near ties, and the result's
+    assert bool(((out.double() - want).abs()[clear] <= 2.0 ** -7 * want.abs().max()).all())

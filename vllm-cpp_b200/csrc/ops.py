@@ -1242,12 +1242,17 @@ MOE_TILE_ROWS = (16, 64, 128)       # heights of the expert products' tiles: sho
 
 def moe_tile_rows(n_tokens: int, top: int, n_experts: int, tensor_cores: bool = False) -> int:
     """The tile height for a step: 64 rows once an expert gets that many tokens on average, else 16.  ``tensor_cores``
-    (bfloat16, both products' widths multiples of 8): 128 rows, the tcgen05 products, from 16 tokens an expert on (4 of 32
+    (bfloat16 that moe_tensor_tiles finds fit): 128 rows, the tcgen05 products, from 16 tokens an expert on (4 of 32
     experts of 2,048, width 4,096, both products: 128 tokens 277 us against 338 with 16 rows, 256 tokens 281 against 512, 512 tokens 292
     against 629 with 64)."""
     if tensor_cores and n_tokens * top >= 16 * n_experts:
         return 128
     return 64 if n_tokens * top >= 64 * n_experts else 16
+
+
+def moe_tensor_tiles(x: torch.Tensor, hidden: int, ff: int) -> bool:
+    """Whether the tcgen05 products can take the tokens' rows ``x`` and matrices of ``hidden`` and ``ff``: bfloat16 in rows of 16-byte pieces."""
+    return x.dtype == torch.bfloat16 and hidden % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
 
 
 def moe_max_tiles(n_tokens: int, top: int, n_experts: int, tm: int) -> int:
