@@ -1768,7 +1768,7 @@ def rufisun_kernels(z, peaks):
     w1, w2 = rnd(E, ef, h, scale=0.02), rnd(E, 2 * ef, h, scale=0.02)
     for t in (8, 64, 2048):
         pairs, xs = t * top, rnd(t, h)
-        tm = ops.moe_tile_rows(t, top, E, tensor_cores=ops.moe_tensor_tiles(xs, h, ef))
+        tm = ops.moe_tile_rows(t, top, E, ops.moe_tensor_tiles(xs, h, ef), h * ef)
         tiles = ops.moe_max_tiles(t, top, E, tm)
         ids = torch.stack([torch.randperm(E, device=dev)[:top] for _ in range(t)]).to(torch.int32).contiguous()
         ints = [torch.empty(n, dtype=torch.int32, device=dev) for n in (pairs, pairs, tiles, tiles, tiles, 4)]

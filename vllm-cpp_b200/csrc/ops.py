@@ -1240,14 +1240,19 @@ def qk_head_rope_cache_write(proj: torch.Tensor, q_off: int, k_off: int, v_off: 
 MOE_TILE_ROWS = (16, 64, 128)       # heights of the expert products' tiles: short for steps of few tokens; 128: tcgen05, bfloat16
 
 
-def moe_tile_rows(n_tokens: int, top: int, n_experts: int, tensor_cores: bool = False) -> int:
-    """The tile height for a step: 64 rows once an expert gets that many tokens on average, else 16.  ``tensor_cores``
-    (bfloat16 that moe_tensor_tiles finds fit): 128 rows, the tcgen05 products, from 16 tokens an expert on (4 of 32
-    experts of 2,048, width 4,096, both products: 128 tokens 277 us against 338 with 16 rows, 256 tokens 281 against 512, 512 tokens 292
-    against 629 with 64)."""
-    if tensor_cores and n_tokens * top >= 16 * n_experts:
-        return 128
-    return 64 if n_tokens * top >= 64 * n_experts else 16
+def moe_tile_rows(n_tokens: int, top: int, n_experts: int, tensor_cores: bool = False, expert_size: Optional[int] = None) -> int:
+    """The tile height for a step: 64 rows once an expert gets that many tokens on average, else 16.  ``tensor_cores`` (bfloat16 that
+    moe_tensor_tiles finds fit): 128 rows, the tcgen05 products, from 16 tokens an expert on (both products, us: 32 experts of 2,048,
+    width 4,096, 4 choices, 128 tokens 274 against 344 with 16 rows, 512 tokens 292 against 656 with 64), if the step's products are large
+    enough for a CTA of 128 x 256 sums to be worth its start: ``expert_size``, the elements of an expert's matrix (width times size;
+    None: large), times the pairs at least 4e8.  At that product the two heights cross for every shape measured (8 experts of 1,024, width 2,048, 2
+    choices: 64 tokens, 2.7e8, 46.9 against 40.6, 80 tokens, 3.4e8, 46.9 against 49.4; 32 of 256, width 1,024, 4 choices: 256 tokens, 2.7e8, 31.1 against
+    30.5, 384, 4.0e8, 31.6 against 33.1; 4 of 512, width 1,024: 800 tokens, 4.2e8, 36.1 against 31.7; 3 of 96, width 64: 22 against 8).  Smaller
+    steps stay at 16 rows: tiles of 64 of so few CTAs are slower (4 of 512, width 1,024, 512 tokens: 42.7 against 29.4)."""
+    pairs = n_tokens * top
+    if tensor_cores and pairs >= 16 * n_experts:
+        return 128 if expert_size is None or pairs * expert_size >= 4e8 else 16
+    return 64 if pairs >= 64 * n_experts else 16
 
 
 def moe_tensor_tiles(x: torch.Tensor, hidden: int, ff: int) -> bool:

@@ -125,7 +125,7 @@ class RoutedExperts(FeedForward):
         n = x.shape[0]
         mark = ws.mark()
         pairs = n * self.top
-        tm = ops.moe_tile_rows(n, self.top, self.E, tensor_cores=ops.moe_tensor_tiles(x, self.hidden, self.ff))
+        tm = ops.moe_tile_rows(n, self.top, self.E, ops.moe_tensor_tiles(x, self.hidden, self.ff), self.hidden * self.ff)
         tiles = ops.moe_max_tiles(n, self.top, self.E, tm)
         ids = ws.take((n, self.top), torch.int32)
         weights = ws.take((n, self.top), torch.float32)
