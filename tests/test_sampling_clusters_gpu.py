@@ -85,7 +85,7 @@ def test_whole_rows(vocab):
             assert e[g] > 0
 
 
-# slabs with ids, of a run's 16: 3, 15, 14, 15, all
+# slabs with ids: 3 and 15 of a short row's 32, 14, 15 and all of a run's 16
 @pytest.mark.parametrize("vocab", [384, 1800, 100352, 152064, 65536])
 def test_every_draw_has_an_id(vocab):
     """The largest uniform number that 24 bits give: the draw lies within the last place of the row's sum, in whichever order that was added up."""
@@ -150,6 +150,27 @@ def test_rows_that_are_no_numbers(vocab):
         assert all(0 <= g < vocab for g in out.tolist())
         ops.sample(logits, dev([0.0] * 7, np.float32), u, out.fill_(-7))
         assert all(0 <= g < vocab for g in out.tolist()) and out.tolist()[2] == vocab // 3 and out.tolist()[6] == 1
+
+
+@pytest.mark.parametrize("vocab", [9001, 20000, 70001, 152064])
+def test_rows_do_not_depend_on_the_batch(vocab):
+    """How many CTAs share a row depends on the batch, its draw does not: 1 to 300 rows, which take eight CTAs to one."""
+    from vllm_cpp_b200.csrc import ops
+    gen = torch.Generator(device="cuda").manual_seed(vocab)
+    logits = 2 * torch.randn(300, vocab, device="cuda", generator=gen)
+    logits[5::7] *= 0.01                                                # flat rows: the search by digits
+    u = torch.rand(300, device="cuda", generator=gen)
+    temp, p, k = torch.full((300,), 0.8, device="cuda"), torch.ones(300, device="cuda"), torch.full((300,), -1, dtype=torch.int32, device="cuda")
+    temp[::5] = 0.0
+    p[1::3], k[2::4] = 0.9, 40
+    whole = None
+    for n in (300, 140, 70, 60, 40, 25, 20, 9, 1):
+        drawn, mixed = torch.full((n,), -7, dtype=torch.int32, device="cuda"), torch.full((n,), -7, dtype=torch.int32, device="cuda")
+        ops.sample(logits[:n], temp[:n], u[:n], drawn)
+        ops.sample_all(logits[:n], temp[:n], u[:n], p[:n], k[:n], mixed)
+        whole = whole or (drawn, mixed)
+        assert torch.equal(drawn, whole[0][:n]) and torch.equal(mixed, whole[1][:n]), n
+        assert bool(((mixed >= 0) & (mixed < vocab)).all())
 
 
 @pytest.mark.parametrize("vocab", [997, 70001])

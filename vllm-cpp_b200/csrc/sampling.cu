@@ -1,4 +1,4 @@
-// Sampling on the device, one CTA or a cluster of eight per logits row, so that only token ids cross
+// Sampling on the device, one CTA or a cluster of up to eight per logits row, so that only token ids cross
 // to the host.  The reference samples on the CPU after copying the whole row
 // (src/core/engine.cpp:209-214, src/sampler/sampler.cpp:23-79).
 //
@@ -19,26 +19,46 @@
 
 namespace cg = cooperative_groups;
 
-// A row is read by the CTAs of a cluster, each a contiguous run of ids (a multiple of 128 long).  One SM takes 32 us for the 608 KB of
-// 152,064 logits (64 rows at once, greedy); eight SMs take an eighth each, 13 us.  How many is decided by
-// the vocabulary alone, so that a row's sums (whose order follows the cut) do not depend on the batch it is in.  Below 16,384
-// ids a row is a few round trips to memory for one CTA too, and the cluster's barriers would cost more than they save.
-#define SAMPLE_THREADS 512
-static inline int sample_ctas(int vocab) { return vocab >= 65536 ? 8 : vocab >= 16384 ? 4 : 1; }
-__device__ __forceinline__ int sample_run(int vocab, int ctas) { return ((vocab + ctas - 1) / ctas + 127) & ~127; }
+// A row is cut into runs of ids (a multiple of 128 long) and a run into slabs: by the vocabulary alone, so that a row's sums, whose
+// order follows the cut, do not depend on the batch it is in.  Below 16,384 ids a row is a few round trips to memory for one
+// CTA too and is one run.
+#define SAMPLE_MAX_RUNS 8
+#define SAMPLE_MAX_SLABS 128           // of a row
+#define FILT_THREADS 1024
+#define FILT_WARPS 32
+static inline int sample_runs(int vocab) { return vocab >= 65536 ? 8 : vocab >= 16384 ? 4 : 1; }
+__host__ __device__ constexpr int sample_run(int vocab, int runs) { return ((vocab + runs - 1) / runs + 127) & ~127; }
+__host__ __device__ constexpr int sample_slabs(int runs) { return runs == 1 ? 32 : 16; }    // of a run
+
+// The runs of a row are dealt out over the CTAs of a cluster, as many as `room` CTAs on the device allow: few rows wait for what one SM
+// takes in, many fill the device with a CTA each and would only wait for the clusters' starts and barriers.
+// (The logarithm to base 2 of their number: the kernels know the runs when they are compiled and shift by this.)
+static inline int sample_ctas_log(int vocab, int n_rows, int room) {
+    const int runs = sample_runs(vocab);
+    int lc = runs == 8 ? 3 : runs == 4 ? 2 : 0;
+    while (lc > 0 && ((long long)n_rows << lc) > room) --lc;
+    return lc;
+}
+// Between the CTAs of a row.
+__device__ __forceinline__ void row_sync(int ctas) {
+    if (ctas == 1) __syncthreads();
+    else cg::this_cluster().sync();
+}
+template <typename T> __device__ __forceinline__ T* row_peer(T* p, int rank, int ctas) { return ctas == 1 ? p : cg::this_cluster().map_shared_rank(p, rank); }
 
 template <typename... KArgs, typename... Args>
-static int sample_launch(void (*kernel)(KArgs...), int n_rows, int ctas, cudaStream_t stream, Args... args) {
+static int sample_launch(void (*kernel)(KArgs...), int threads, int n_rows, int lc, cudaStream_t stream, Args... args) {
+    const int ctas = 1 << lc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_rows * ctas);
-    cfg.blockDim = SAMPLE_THREADS;
+    cfg.blockDim = threads;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ctas > 1 ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
     return e != cudaSuccess ? (int)e : vcb_last_error();
 }
@@ -71,21 +91,24 @@ __device__ __forceinline__ void argmax_combine(float& bv, int& bi, float ov, int
     if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
 }
 
+template <int RUNS>
 __device__ __forceinline__ void
 sample_row(const float* __restrict__ logits, int ld, int vocab, const float* __restrict__ temperature,
-           const float* __restrict__ uniform, int* __restrict__ out, int ctas) {
-    __shared__ float scratch[33];
+           const float* __restrict__ uniform, int* __restrict__ out, int lc) {
+    __shared__ float own[SAMPLE_MAX_SLABS], slabs[SAMPLE_MAX_SLABS];      // [runs of this CTA][slabs]
     __shared__ float sval[32];
     __shared__ int sidx[32];
     __shared__ int winner;
-    __shared__ float cta_max, cta_sum;                     // read by the row's other CTAs
+    __shared__ float cta_max, run_sum[SAMPLE_MAX_RUNS];    // read by the row's other CTAs
     __shared__ int cta_idx;
-    cg::cluster_group cluster = cg::this_cluster();
-    const int row = blockIdx.x / ctas, rank = blockIdx.x % ctas;
+    const int ctas = RUNS > 1 ? 1 << lc : 1, per_log = RUNS > 1 ? (RUNS == 8 ? 3 : 2) - lc : 0, per = 1 << per_log;      // per: runs of a CTA
+    const int row = RUNS > 1 ? blockIdx.x >> lc : blockIdx.x, rank = RUNS > 1 ? blockIdx.x & (ctas - 1) : 0;
     const float* l = logits + (size_t)row * ld;
     const float temp = temperature[row];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int run = sample_run(vocab, ctas), first = min(vocab, rank * run), last = min(vocab, first + run);
+    const int run = sample_run(vocab, RUNS), first = min(vocab, rank * per * run), last = min(vocab, first + per * run);
+    constexpr int per_run = sample_slabs(RUNS);
+    const int slab = ((run + per_run - 1) / per_run + 127) & ~127;
     const bool aligned = (((uintptr_t)l) & 15) == 0;       // runs and slabs start at multiples of 128
 
     // The largest logit and its lowest id; the maximum is also softmax's shift.
@@ -137,29 +160,27 @@ sample_row(const float* __restrict__ logits, int ld, int vocab, const float* __r
         }
         if (lane == 0) { cta_max = bv; cta_idx = bi; }
     }
-    cluster.sync();
+    row_sync(ctas);
     float lmax = -INFINITY;
     int imax = vocab;
-    for (int c = 0; c < ctas; ++c) argmax_combine(lmax, imax, *cluster.map_shared_rank(&cta_max, c), *cluster.map_shared_rank(&cta_idx, c));
+    for (int c = 0; c < ctas; ++c) argmax_combine(lmax, imax, *row_peer(&cta_max, c, ctas), *row_peer(&cta_idx, c, ctas));
     if (imax >= vocab) imax = 0;
     if (temp <= 0.0f) {                                    // the whole cluster: a row has one temperature
         if (rank == 0 && threadIdx.x == 0) out[row] = imax;
-        cluster.sync();                                    // nobody leaves while its maximum is being read
+        if (ctas > 1) row_sync(ctas);                      // nobody leaves while its maximum is being read
         return;
     }
 
-    // e_i = exp((l_i - max) / T).  Every warp owns a contiguous slab of ids, so the warps' sums, taken in the
-    // order of the warps, follow the order of the ids; inside its slab a warp reads rows of 128 ids (a float4
+    // e_i = exp((l_i - max) / T).  A warp sums a contiguous slab of a run's ids, so the slabs' sums, taken in their
+    // order, follow the order of the ids; inside its slab a warp reads rows of 128 ids (a float4
     // a lane, four rows in flight), each lane adding up what it reads.  The slab that holds the draw is then
     // walked once more by its warp, row by row in the order of the ids.
     const float inv_t = 1.0f / temp;
     const float xmax = temp != 1.0f ? lmax * inv_t : lmax;
     const bool scaled = temp != 1.0f;
     auto weight = [&](float v) { return expf((scaled ? v * inv_t : v) - xmax); };
-    const int slab = ((run + nwarps - 1) / nwarps + 127) & ~127;
-    const int lo = min(last, first + warp * slab), hi = min(last, lo + slab);
-    // the four weights of this lane in the row that starts at id `base` (zero beyond the slab)
-    auto row_weights = [&](int base, float (&e)[4]) {
+    // the four weights of this lane in the row that starts at id `base` of a slab that ends at `hi` (zero beyond it)
+    auto row_weights = [&](int base, int hi, float (&e)[4]) {
         const int i = base + lane * 4;
         if (aligned && i + 3 < hi) {
             const float4 v = *reinterpret_cast<const float4*>(l + i);
@@ -169,8 +190,16 @@ sample_row(const float* __restrict__ logits, int ld, int vocab, const float* __r
             for (int k = 0; k < 4; ++k) e[k] = i + k < hi ? weight(l[i + k]) : 0.0f;
         }
     };
-    float local = 0.0f;
-    {
+    // [lo, hi): slab v of this CTA's
+    auto slab_ids = [&](int v, int& lo, int& hi) {
+        const int run_first = min(last, first + v / per_run * run), run_last = min(last, run_first + run);
+        lo = min(run_last, run_first + v % per_run * slab);
+        hi = min(run_last, lo + slab);
+    };
+    for (int v0 = warp; v0 < per * per_run; v0 += nwarps) {
+        int lo, hi;
+        slab_ids(v0, lo, hi);
+        float local = 0.0f;
         constexpr int U = 4;
         int base = lo;
         if (aligned) {
@@ -181,53 +210,74 @@ sample_row(const float* __restrict__ logits, int ld, int vocab, const float* __r
 #pragma unroll
                 for (int u = 0; u < U; ++u) local += (weight(v[u].x) + weight(v[u].y)) + (weight(v[u].z) + weight(v[u].w));
             }
+            if (base + 2 * 128 <= hi) {
+                const float4 a = *reinterpret_cast<const float4*>(l + base + lane * 4), b = *reinterpret_cast<const float4*>(l + base + 128 + lane * 4);
+                local += (weight(a.x) + weight(a.y)) + (weight(a.z) + weight(a.w));
+                local += (weight(b.x) + weight(b.y)) + (weight(b.z) + weight(b.w));
+                base += 2 * 128;
+            }
         }
         for (; base < hi; base += 128) {
             float e[4];
-            row_weights(base, e);
+            row_weights(base, hi, e);
             local += (e[0] + e[1]) + (e[2] + e[3]);
         }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);      // the slab's sum, in all lanes
-    if (lane == 0) scratch[warp] = local;
+        for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
+        if (lane == 0) own[v0] = local;
+    }
     __syncthreads();
-    if (warp == 0) {
-        float w = lane < nwarps ? scratch[lane] : 0.0f;
+    if (warp < per) {                                      // a run a warp
+        float w = lane < per_run ? own[warp * per_run + lane] : 0.0f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float y = __shfl_up_sync(0xffffffffu, w, o);
             if (lane >= o) w += y;
         }
-        scratch[lane] = w;                 // inclusive sums of the slabs
+        if (lane < per_run) slabs[warp * per_run + lane] = w;              // inclusive sums of the run's slabs
         // The run's sum is that of its last slab with ids: an empty slab behind it adds nothing, but its sum is another tree of the same
         // numbers and may be a unit in the last place larger, and a draw between the two would lie in no slab.
-        if (lane == (last > first ? (last - first - 1) / slab : 0)) cta_sum = w;
+        const int ids = min(last, first + (warp + 1) * run) - min(last, first + warp * run);
+        if (lane == (ids > 0 ? (ids - 1) / slab : 0)) run_sum[warp] = w;
     }
-    if (threadIdx.x == 0) winner = nwarps;
-    cluster.sync();
-    float before_cta = 0.0f, total = 0.0f;                 // the runs before this one; all
-    for (int c = 0; c < ctas; ++c) {
-        if (c == rank) before_cta = total;
-        total += *cluster.map_shared_rank(&cta_sum, c);
-    }
-    cluster.sync();                                        // the other CTAs' sums are read: from here on each is alone
+    if (threadIdx.x == 0) winner = per * per_run;
+    row_sync(ctas);
+    const float mine = lane < RUNS ? *row_peer(&run_sum[lane & (per - 1)], lane >> per_log, ctas) : 0.0f;      // a run's sum a lane
+    float total = 0.0f;
+#pragma unroll
+    for (int c = 0; c < RUNS; ++c) total += __shfl_sync(0xffffffffu, mine, c);
     const float target = uniform[row] * total;
+    // the run that holds the draw: the first whose inclusive sum exceeds it
+    int held = -1;
+    float before_run = 0.0f, upto_run = 0.0f;
+#pragma unroll
+    for (int c = 0; c < RUNS; ++c) {
+        const float next = upto_run + __shfl_sync(0xffffffffu, mine, c);
+        if (held < 0 && target < next) { held = c; before_run = upto_run; }
+        upto_run = next;
+    }
+    if (ctas > 1) row_sync(ctas);                          // the other CTAs' sums are read: from here on each is alone
     if (!(target < total)) {                               // u * total >= total after rounding: the last id
         if (rank == 0 && threadIdx.x == 0) out[row] = vocab - 1;
         return;
     }
-    // the run that holds the draw: the first whose inclusive sum exceeds it
-    if (!(target < before_cta + cta_sum) || (rank > 0 && target < before_cta)) return;
-    const float incl = before_cta + scratch[warp];
-    if (lane == 0 && hi > lo && target < incl) atomicMin(&winner, warp);
+    if (held >> per_log != rank) return;
+    const int v_first = (held & (per - 1)) * per_run;
+    if ((int)threadIdx.x < per_run) {
+        int lo, hi;
+        slab_ids(v_first + threadIdx.x, lo, hi);
+        if (hi > lo && target < before_run + slabs[v_first + threadIdx.x]) atomicMin(&winner, v_first + (int)threadIdx.x);
+    }
     __syncthreads();
-    if (warp != winner) return;                            // there is one: the last slab that has ids ends at the run's sum
-    float c = incl - local;                      // the sum before this slab
+    if (warp != 0) return;
+    int lo, hi;
+    slab_ids(winner, lo, hi);                              // there is one: the last slab that has ids ends at the run's sum
+    const float incl = before_run + slabs[winner];
+    float c = incl - own[winner];                // the sum before this slab
     int tok = hi - 1;                            // if rounding keeps the walk's sums below the draw: the slab's last id
     for (int base = lo; base < hi; base += 128) {
         float e[4];
-        row_weights(base, e);
+        row_weights(base, hi, e);
         const float p1 = e[0], p2 = p1 + e[1], p3 = p2 + e[2], p4 = p3 + e[3];
         float upto = p4;                         // inclusive sum of the lanes' four
 #pragma unroll
@@ -254,18 +304,28 @@ sample_row(const float* __restrict__ logits, int ld, int vocab, const float* __r
     if (lane == 0) out[row] = tok;
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+template <int RUNS, int THREADS>
+__global__ void __launch_bounds__(THREADS, 2)
 sample_kernel(const float* __restrict__ logits, int ld, int vocab, const float* __restrict__ temperature,
-              const float* __restrict__ uniform, int* __restrict__ out, int ctas) {
-    sample_row(logits, ld, vocab, temperature, uniform, out, ctas);
+              const float* __restrict__ uniform, int* __restrict__ out, int lc) {
+    sample_row<RUNS>(logits, ld, vocab, temperature, uniform, out, lc);
 }
 
 VCB_EXPORT int vcb_sample(const float* logits, int ld, int vocab, const float* temperature,
                           const float* uniform, int* out, int n_rows, void* stream) {
     if (n_rows <= 0) return 0;
     if (vocab <= 0 || ld < vocab) return VCB_ERR_BAD_ARG;
-    const int ctas = sample_ctas(vocab);
-    return sample_launch(sample_kernel, n_rows, ctas, (cudaStream_t)stream, logits, ld, vocab, temperature, uniform, out, ctas);
+    // Few rows of many ids in clusters of CTAs of 512 threads (us, greedy / a draw, of 152,064 ids: 8 rows in eight CTAs 6.8 / 15.6, in one
+    // of 1,024 threads 10.0 / 26.4; 64 rows in four 9.5 / 22.4, in one 10.8 / 27.0); more rows, and shorter ones, a CTA of 1,024 threads each (256
+    // rows 28 / 62, in eight CTAs 43 / 78; 64 rows of 32,000 5.3 / 10.5, in four CTAs 6.7 / 12.1).
+    const int runs = sample_runs(vocab);
+    const bool few = runs > 1 && n_rows <= (runs == 8 ? 64 : 24);
+    const int lc = few ? sample_ctas_log(vocab, n_rows, 256) : 0;
+#define SAMPLE(R, T) sample_launch(sample_kernel<R, T>, T, n_rows, lc, (cudaStream_t)stream, logits, ld, vocab, temperature, uniform, out, lc)
+    if (runs == 8) return few ? SAMPLE(8, 512) : SAMPLE(8, 1024);
+    if (runs == 4) return few ? SAMPLE(4, 512) : SAMPLE(4, 1024);
+    return SAMPLE(1, 1024);
+#undef SAMPLE
 }
 
 // --------------------------------------------------------- top-k / top-p
@@ -290,23 +350,24 @@ VCB_EXPORT int vcb_sample(const float* logits, int ld, int vocab, const float* t
 // sum is its count times those plus a whole number of units in the last place, kept as two counters of ten bits each (2^20 ids
 // fit 32 bits); bins are added up in double.
 //
-// 64 rows of 152,064 (temperature 0.8, top-k 50 and top-p 0.9): digits of four bits, one CTA a row, 39 passes bound by sixteen comparisons an
-// id, 1,549 us; digits of ten bits in clusters 268 us (bound by three shared-memory counters an id and by eight passes); the list 114 us.
-// (Flat rows, top-p 0.9 of logits of deviation 2: 374 us by digits.)
+// 64 rows of 152,064 (temperature 0.8, top-k 50 and top-p 0.9): digits of four bits in one CTA a row, 39 passes bound by sixteen comparisons an
+// id, 1,549 us; the list 43 us, bound by the three passes' loads, exponentials and a counter an id.  Flat rows (top-p 0.9 of logits of deviation 2) by
+// digits of ten bits 103 us, bound by three counters an id and eight passes; equal logits, whose counters all lie in one bin, 190 us.
 // e is kept in scratch memory supplied by the caller: rows * vocab floats.
 enum { COND_COUNT_GE = 0, COND_SUM_GE = 1, COND_SUM_GT = 2 };
-constexpr int FILT_BINS = 1024, FILT_MINE = FILT_BINS / SAMPLE_THREADS;       // bins of a digit; of a thread
+constexpr int FILT_BINS = 1024;                            // of a digit, one a thread
+static_assert(FILT_BINS == FILT_THREADS, "a bin a thread");
 
 __device__ __forceinline__ unsigned long long filt_key(float e, int id) {
     return ((unsigned long long)__float_as_uint(e) << 20) | (unsigned long long)(0xFFFFF - id);
 }
 
-constexpr int FILT_LIST = 4096, FILT_PER = FILT_LIST / SAMPLE_THREADS;
+constexpr int FILT_LIST = 4096, FILT_PER = FILT_LIST / FILT_THREADS;
 
 struct FiltShared {
     unsigned long long list[FILT_LIST];                    // the first CTA's: keys
     int listed;
-    double cta_total;
+    double run_total[SAMPLE_MAX_RUNS];
     unsigned count[FILT_BINS], low[FILT_BINS], high[FILT_BINS];               // read by the row's other CTAs
     double wsum[32], above_sum, at_sum;
     unsigned wcnt[32], above_cnt, at_cnt;
@@ -314,83 +375,87 @@ struct FiltShared {
     float cta_max;
 };
 
-// What the CTAs of a row share; a thread's bins are 1023 - (2 t), 1023 - (2 t + 1): falling weights.
+// What the CTAs of a row share; a thread's bin is 1023 - t: falling weights.
 struct FiltRow {
     const float* e;
     int first, last, ctas;
     bool vec;
     FiltShared* sh;
 
-    template <typename F> __device__ __forceinline__ void for_each(F f) const {
+    template <typename F> __device__ __forceinline__ void for_each(F f) const { for_each(first, last, f); }
+    template <typename F> __device__ __forceinline__ void for_each(int first, int last, F f) const {
         if (vec) {
             const float4* e4 = reinterpret_cast<const float4*>(e + first);
             const int nvec = (last - first) >> 2;
             constexpr int U = 4;
             int i = threadIdx.x;
-            for (; i + (U - 1) * SAMPLE_THREADS < nvec; i += U * SAMPLE_THREADS) {
+            for (; i + (U - 1) * FILT_THREADS < nvec; i += U * FILT_THREADS) {
                 float4 v[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) v[u] = e4[i + u * SAMPLE_THREADS];
+                for (int u = 0; u < U; ++u) v[u] = e4[i + u * FILT_THREADS];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int id = first + 4 * (i + u * SAMPLE_THREADS);
+                    const int id = first + 4 * (i + u * FILT_THREADS);
                     f(v[u].x, id); f(v[u].y, id + 1); f(v[u].z, id + 2); f(v[u].w, id + 3);
                 }
             }
-            for (; i < nvec; i += SAMPLE_THREADS) {
+            for (; i < nvec; i += FILT_THREADS) {
                 const float4 v = e4[i];
                 const int id = first + 4 * i;
                 f(v.x, id); f(v.y, id + 1); f(v.z, id + 2); f(v.w, id + 3);
             }
-            for (int j = first + (nvec << 2) + threadIdx.x; j < last; j += SAMPLE_THREADS) f(e[j], j);
+            for (int j = first + (nvec << 2) + threadIdx.x; j < last; j += FILT_THREADS) f(e[j], j);
         } else {
-            for (int i = first + threadIdx.x; i < last; i += SAMPLE_THREADS) f(e[i], i);
+            for (int i = first + threadIdx.x; i < last; i += FILT_THREADS) f(e[i], i);
         }
     }
     __device__ __forceinline__ void clear() const {
-        for (int i = threadIdx.x; i < FILT_BINS; i += SAMPLE_THREADS) { sh->count[i] = 0; sh->low[i] = 0; sh->high[i] = 0; }
+        for (int i = threadIdx.x; i < FILT_BINS; i += FILT_THREADS) { sh->count[i] = 0; sh->low[i] = 0; sh->high[i] = 0; }
         __syncthreads();
     }
-    __device__ __forceinline__ void add(int bin, unsigned rest) const {       // rest: the key's weight bits below the digit, at most 20
-        atomicAdd(&sh->count[bin], 1u);
-        if (rest & 1023u) atomicAdd(&sh->low[bin], rest & 1023u);
-        if (rest >> 10) atomicAdd(&sh->high[bin], rest >> 10);
+    // An id's counters.  Neighbouring ids of one bin are added up in registers first: in flat rows most are in few bins, and the
+    // atomics of a bin take turns (64 rows of 152,064 equal logits: 760 us with an atomic an id, 190 so).
+    struct Bin { int at; unsigned n, lo, hi; };
+    __device__ __forceinline__ void flush(Bin& b) const {
+        if (b.n) atomicAdd(&sh->count[b.at], b.n);
+        if (b.lo) atomicAdd(&sh->low[b.at], b.lo);
+        if (b.hi) atomicAdd(&sh->high[b.at], b.hi);
     }
-    // This thread's bins over all CTAs; ends with the counters free to be cleared.  value(bin): the weight's leading bits.
-    template <typename V>
-    __device__ __forceinline__ void collect(unsigned (&cnt)[FILT_MINE], double (&sum)[FILT_MINE], V value) const {
-        cg::cluster_group cluster = cg::this_cluster();
-        cluster.sync();
-#pragma unroll
-        for (int j = 0; j < FILT_MINE; ++j) {
-            const int bin = FILT_BINS - 1 - (threadIdx.x * FILT_MINE + j);
-            unsigned c = 0, lo = 0, hi = 0;
-            for (int r = 0; r < ctas; ++r) {
-                c += *cluster.map_shared_rank(&sh->count[bin], r);
-                lo += *cluster.map_shared_rank(&sh->low[bin], r);
-                hi += *cluster.map_shared_rank(&sh->high[bin], r);
-            }
-            const unsigned bits = value(bin);
-            const double at = (double)__uint_as_float(bits), unit = (double)__uint_as_float(bits + 1) - at;
-            cnt[j] = c;
-            sum[j] = c ? (double)c * at + ((double)hi * 1024.0 + (double)lo) * unit : 0.0;
+    __device__ __forceinline__ void add(Bin& b, int bin, unsigned rest) const {       // rest: the key's weight bits below the digit, at most 20
+        if (bin != b.at) {
+            flush(b);
+            b = Bin{bin, 0u, 0u, 0u};
         }
-        cluster.sync();
+        b.n += 1;
+        b.lo += rest & 1023u;
+        b.hi += rest >> 10;
+    }
+    // This thread's bin over all CTAs; ends with the counters free to be cleared.  value(bin): the weight's leading bits.
+    template <typename V>
+    __device__ __forceinline__ void collect(unsigned& cnt, double& sum, V value) const {
+        row_sync(ctas);
+        const int bin = FILT_BINS - 1 - threadIdx.x;
+        unsigned c = 0, lo = 0, hi = 0;
+        for (int r = 0; r < ctas; ++r) {
+            c += *row_peer(&sh->count[bin], r, ctas);
+            lo += *row_peer(&sh->low[bin], r, ctas);
+            hi += *row_peer(&sh->high[bin], r, ctas);
+        }
+        const unsigned bits = value(bin);
+        const double at = (double)__uint_as_float(bits), unit = (double)__uint_as_float(bits + 1) - at;
+        cnt = c;
+        sum = c ? (double)c * at + ((double)hi * 1024.0 + (double)lo) * unit : 0.0;
+        row_sync(ctas);
     }
 };
 
 // The first of the row's bins (largest weights first) at which the running count or sum, on top of above_*, meets the bound.
 // Sets sh.chosen, sh.above_* (before that bin) and sh.at_* (with it).
 template <int COND>
-__device__ __forceinline__ void filt_choose(FiltShared& sh, const unsigned (&cnt)[FILT_MINE], const double (&sum)[FILT_MINE],
-                                            unsigned above_cnt, double above_sum, double bound) {
+__device__ __forceinline__ void filt_choose(FiltShared& sh, unsigned cnt, double sum, unsigned above_cnt, double above_sum, double bound) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned c = 0;
-    double s = 0.0;
-#pragma unroll
-    for (int j = 0; j < FILT_MINE; ++j) { c += cnt[j]; s += sum[j]; }
-    unsigned ci = c;
-    double si = s;
+    unsigned ci = cnt;
+    double si = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const unsigned cy = __shfl_up_sync(0xffffffffu, ci, o);
@@ -404,24 +469,12 @@ __device__ __forceinline__ void filt_choose(FiltShared& sh, const unsigned (&cnt
     unsigned cb = above_cnt;
     double sb = above_sum;
     for (int w = 0; w < warp; ++w) { cb += sh.wcnt[w]; sb += sh.wsum[w]; }
-    cb += ci - c;
-    sb += si - s;                                          // exact enough: doubles of at most 2^20 terms
-    int hit = FILT_BINS, lowest = -1;
-    unsigned hit_cb = 0, hit_c = 0, low_cb = 0, low_c = 0;
-    double hit_sb = 0.0, hit_s = 0.0, low_sb = 0.0, low_s = 0.0;
-#pragma unroll
-    for (int j = 0; j < FILT_MINE; ++j) {
-        const unsigned c1 = cb + cnt[j];
-        const double s1 = sb + sum[j];
-        const bool ok = COND == COND_COUNT_GE ? (double)c1 >= bound : COND == COND_SUM_GE ? s1 >= bound : s1 > bound;
-        const int at = threadIdx.x * FILT_MINE + j;
-        if (cnt[j]) {
-            if (ok && hit == FILT_BINS) { hit = at; hit_cb = cb; hit_c = c1; hit_sb = sb; hit_s = s1; }
-            lowest = at; low_cb = cb; low_c = c1; low_sb = sb; low_s = s1;
-        }
-        cb = c1;
-        sb = s1;
-    }
+    cb += ci - cnt;
+    sb += si - sum;                                        // exact enough: doubles of at most 2^20 terms
+    const unsigned c1 = cb + cnt;
+    const double s1 = sb + sum;
+    const bool ok = COND == COND_COUNT_GE ? (double)c1 >= bound : COND == COND_SUM_GE ? s1 >= bound : s1 > bound;
+    int hit = cnt && ok ? (int)threadIdx.x : FILT_BINS;
     if (hit < FILT_BINS) atomicMin(&sh.chosen, hit);
     __syncthreads();
     int chosen = sh.chosen;
@@ -431,20 +484,19 @@ __device__ __forceinline__ void filt_choose(FiltShared& sh, const unsigned (&cnt
         __syncthreads();
         if (threadIdx.x == 0) sh.chosen = -1;
         __syncthreads();
-        if (lowest >= 0) atomicMax(&sh.chosen, lowest);
+        if (cnt) atomicMax(&sh.chosen, (int)threadIdx.x);
         __syncthreads();
         chosen = sh.chosen;
-        hit = lowest; hit_cb = low_cb; hit_c = low_c; hit_sb = low_sb; hit_s = low_s;
+        hit = cnt ? (int)threadIdx.x : -1;
     }
-    if (chosen >= 0 && hit == chosen) { sh.above_cnt = hit_cb; sh.at_cnt = hit_c; sh.above_sum = hit_sb; sh.at_sum = hit_s; }
+    if (chosen >= 0 && hit == chosen) { sh.above_cnt = cb; sh.at_cnt = c1; sh.above_sum = sb; sh.at_sum = s1; }
     __syncthreads();
 }
 
-// The largest key T for which the condition holds, counting only ids with key >= floor_key; cnt1, sum1: this thread's bins of
+// The largest key T for which the condition holds, counting only ids with key >= floor_key; cnt1, sum1: this thread's bin of
 // the first digit, of those ids.  On return sh.at_* are count(T) and sum(T), `shift` the bits of T that were not needed.
 template <int COND>
-__device__ unsigned long long filt_search(const FiltRow& row, const unsigned (&cnt1)[FILT_MINE], const double (&sum1)[FILT_MINE],
-                                          unsigned long long floor_key, double bound, int& shift) {
+__device__ unsigned long long filt_search(const FiltRow& row, unsigned cnt1, double sum1, unsigned long long floor_key, double bound, int& shift) {
     FiltShared& sh = *row.sh;
     filt_choose<COND>(sh, cnt1, sum1, 0u, 0.0, bound);
     unsigned long long prefix = (unsigned long long)(FILT_BINS - 1 - max(sh.chosen, 0));
@@ -455,15 +507,17 @@ __device__ unsigned long long filt_search(const FiltRow& row, const unsigned (&c
         shift -= 10;
         const unsigned top = (unsigned)(prefix >> (30 - shift));              // the first digit, of every level
         row.clear();
+        FiltRow::Bin bin{0, 0u, 0u, 0u};
         row.for_each([&](float e, int id) {
             const unsigned bits = __float_as_uint(e);
             if ((bits >> 20) != top) return;
             const unsigned long long key = filt_key(e, id);
             if ((key >> (shift + 10)) != prefix || key < floor_key) return;
-            row.add((int)((key >> shift) & (FILT_BINS - 1)), shift > 20 ? bits & ((1u << (shift - 20)) - 1) : 0u);
+            row.add(bin, (int)((key >> shift) & (FILT_BINS - 1)), shift > 20 ? bits & ((1u << (shift - 20)) - 1) : 0u);
         });
-        unsigned cnt[FILT_MINE];
-        double sum[FILT_MINE];
+        row.flush(bin);
+        unsigned cnt;
+        double sum;
         const int level = shift;
         row.collect(cnt, sum, [&](int bin) { return (unsigned)((((prefix << 10) | (unsigned)bin) << level) >> 20); });
         filt_choose<COND>(sh, cnt, sum, above_cnt, above_sum, bound);
@@ -477,12 +531,12 @@ __device__ __forceinline__ int filt_draw(FiltShared& sh, int n, int vocab, int k
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int size = 2;
     while (size < n) size <<= 1;
-    for (int i = n + threadIdx.x; i < size; i += SAMPLE_THREADS) sh.list[i] = 0ull;        // below every key: ids are below 0xFFFFF
+    for (int i = n + threadIdx.x; i < size; i += FILT_THREADS) sh.list[i] = 0ull;        // below every key: ids are below 0xFFFFF
     __syncthreads();
     // bitonic, falling
     for (int run = 2; run <= size; run <<= 1)
         for (int step = run >> 1; step > 0; step >>= 1) {
-            for (int t = threadIdx.x; t < size / 2; t += SAMPLE_THREADS) {
+            for (int t = threadIdx.x; t < size / 2; t += FILT_THREADS) {
                 const int i = 2 * t - (t & (step - 1)), j = i + step;
                 const unsigned long long a = sh.list[i], b = sh.list[j];
                 if ((a < b) == ((i & run) == 0)) { sh.list[i] = b; sh.list[j] = a; }
@@ -541,27 +595,26 @@ __device__ __forceinline__ int filt_draw(FiltShared& sh, int n, int vocab, int k
 }
 
 // ALL: rows without top-k and top-p are drawn too (as sample_kernel draws them).
-template <bool ALL>
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+template <int RUNS, bool ALL>
+__global__ void __launch_bounds__(FILT_THREADS)
 sample_filtered_kernel(const float* __restrict__ logits, int ld, int vocab, const float* __restrict__ temperature,
                        const float* __restrict__ uniform, const float* __restrict__ top_p,
-                       const int* __restrict__ top_k, float* __restrict__ scratch, int* __restrict__ out, int ctas) {
+                       const int* __restrict__ top_k, float* __restrict__ scratch, int* __restrict__ out, int lc) {
     __shared__ FiltShared sh;
     __shared__ float red[33];
-    __shared__ double dred[SAMPLE_THREADS / 32];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int row = blockIdx.x / ctas, rank = blockIdx.x % ctas;
+    const int ctas = RUNS > 1 ? 1 << lc : 1, per_log = RUNS > 1 ? (RUNS == 8 ? 3 : 2) - lc : 0, per = 1 << per_log;      // per: runs of a CTA
+    const int row = RUNS > 1 ? blockIdx.x >> lc : blockIdx.x, rank = RUNS > 1 ? blockIdx.x & (ctas - 1) : 0;
     const float temp = temperature[row], p = top_p[row];
     const int k = top_k[row];
     if (!(temp > 0.0f) || !(p < 1.0f || k > 0)) {            // the whole cluster
-        if (ALL) sample_row(logits, ld, vocab, temperature, uniform, out, ctas);
+        if (ALL) sample_row<RUNS>(logits, ld, vocab, temperature, uniform, out, lc);
         return;
     }
     const float* l = logits + (size_t)row * ld;
     float* e = scratch + (size_t)row * vocab;
     const float inv_t = 1.0f / temp;
     const bool scaled = temp != 1.0f;
-    const int run = sample_run(vocab, ctas), first = min(vocab, rank * run), last = min(vocab, first + run);
+    const int run = sample_run(vocab, RUNS), first = min(vocab, rank * per * run), last = min(vocab, first + per * run);
 
     const bool vec = ((((uintptr_t)l) | ((uintptr_t)e)) & 15) == 0;
     FiltRow logit_row{l, first, last, ctas, vec, &sh}, weight_row{e, first, last, ctas, vec, &sh};
@@ -570,8 +623,8 @@ sample_filtered_kernel(const float* __restrict__ logits, int ld, int vocab, cons
     mx = block_max(mx, red);
     if (threadIdx.x == 0) sh.cta_max = mx;
     weight_row.clear();
-    cluster.sync();
-    for (int c = 0; c < ctas; ++c) mx = fmaxf(mx, *cluster.map_shared_rank(&sh.cta_max, c));
+    row_sync(ctas);
+    for (int c = 0; c < ctas; ++c) mx = fmaxf(mx, *row_peer(&sh.cta_max, c, ctas));
     // (The largest has weight 1 even where the difference of two infinities would be no number; what is no number has no weight.)
     // The product is rounded on its own wherever this is inlined: the ids counted and the ids gathered have the same weights.
     auto weight = [&](float v) {
@@ -579,41 +632,48 @@ sample_filtered_kernel(const float* __restrict__ logits, int ld, int vocab, cons
         const float w = x == mx ? 1.0f : expf(x - mx);
         return w <= 1.0f ? w : 0.0f;
     };
-    unsigned cnt[FILT_MINE];
-    double sum[FILT_MINE];
-    double total = 0.0;
-    logit_row.for_each([&](float v, int) {
-        const float w = weight(v);
-        atomicAdd(&sh.count[__float_as_uint(w) >> 20], 1u);
-        total += (double)w;                                  // a thread's ids in their order, then threads, warps and CTAs in theirs
-    });
+    unsigned cnt;
+    double sum;
+    // The row's weight: a run's ids by thread in their order, then threads, warps and runs in theirs, whichever CTA has the run.
+    double* of_warps = reinterpret_cast<double*>(sh.list);                    // [runs][warps]: the list is not begun
+    FiltRow::Bin counted{0, 0u, 0u, 0u};
+    for (int j = 0; j < per; ++j) {
+        const int run_first = min(last, first + j * run);
+        double t = 0.0;
+        logit_row.for_each(run_first, min(last, run_first + run), [&](float v, int) {
+            const float w = weight(v);
+            weight_row.add(counted, (int)(__float_as_uint(w) >> 20), 0u);
+            t += (double)w;
+        });
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    if ((threadIdx.x & 31) == 0) dred[threadIdx.x >> 5] = total;
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if ((threadIdx.x & 31) == 0) of_warps[j * FILT_WARPS + (threadIdx.x >> 5)] = t;
+    }
+    weight_row.flush(counted);
     if (threadIdx.x == 0) sh.listed = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if ((int)threadIdx.x < per) {
         double t = 0.0;
-        for (int w = 0; w < SAMPLE_THREADS / 32; ++w) t += dred[w];
-        sh.cta_total = t;
+        for (int w = 0; w < FILT_WARPS; ++w) t += of_warps[threadIdx.x * FILT_WARPS + w];
+        sh.run_total[threadIdx.x] = t;
     }
     weight_row.collect(cnt, sum, [](int bin) { return (unsigned)bin << 20; });      // (sums at the bins' lower ends: low and high are zero)
-    // sh.cta_total stands until the clusters' next barrier but one
-    total = 0.0;
-    for (int c = 0; c < ctas; ++c) total += *cluster.map_shared_rank(&sh.cta_total, c);
+    // sh.run_total stands until the row's next barrier but one
+    double total = 0.0;
+    for (int c = 0; c < RUNS; ++c) total += *row_peer(&sh.run_total[c & (per - 1)], c >> per_log, ctas);
     if (k > 0 && k < vocab) filt_choose<COND_COUNT_GE>(sh, cnt, sum, 0u, 0.0, (double)k);
     else filt_choose<COND_SUM_GE>(sh, cnt, sum, 0u, 0.0, (p < 1.0f ? (double)p : 1.0) * total);
     if (sh.at_cnt <= FILT_LIST) {
         const unsigned least = (unsigned)(FILT_BINS - 1 - max(sh.chosen, 0)) << 20;
-        int* listed = cluster.map_shared_rank(&sh.listed, 0);
-        unsigned long long* list = cluster.map_shared_rank(sh.list, 0);
+        int* listed = row_peer(&sh.listed, 0, ctas);
+        unsigned long long* list = row_peer(sh.list, 0, ctas);
         logit_row.for_each([&](float v, int id) {
             const float w = weight(v);
             if (__float_as_uint(w) < least) return;
             const int at = atomicAdd(listed, 1);
             if (at < FILT_LIST) list[at] = filt_key(w, id);
         });
-        cluster.sync();
+        row_sync(ctas);
         if (rank != 0) return;
         const int id = filt_draw(sh, min(sh.listed, FILT_LIST), vocab, k, p, uniform[row], total);
         if (threadIdx.x == 0) out[row] = id;
@@ -622,12 +682,14 @@ sample_filtered_kernel(const float* __restrict__ logits, int ld, int vocab, cons
 
     // A thread writes the weights it reads later: no other thread's are needed.
     weight_row.clear();
+    FiltRow::Bin bin{0, 0u, 0u, 0u};
     logit_row.for_each([&](float v, int id) {
         const float w = weight(v);
         e[id] = w;
         const unsigned bits = __float_as_uint(w);
-        weight_row.add((int)(bits >> 20), bits & 0xFFFFFu);
+        weight_row.add(bin, (int)(bits >> 20), bits & 0xFFFFFu);
     });
+    weight_row.flush(bin);
     weight_row.collect(cnt, sum, [](int bin) { return (unsigned)bin << 20; });
 
     unsigned long long floor_key = 0;
@@ -642,12 +704,9 @@ sample_filtered_kernel(const float* __restrict__ logits, int ld, int vocab, cons
         const unsigned above_cnt = sh.above_cnt;
         const double above_sum = sh.above_sum;
         __syncthreads();
-#pragma unroll
-        for (int j = 0; j < FILT_MINE; ++j) {
-            const int bin = FILT_BINS - 1 - (threadIdx.x * FILT_MINE + j);
-            if (bin < digit) { cnt[j] = 0; sum[j] = 0.0; }
-            else if (bin == digit) { cnt[j] = kept_cnt - above_cnt; sum[j] = kept_sum - above_sum; }
-        }
+        const int mine = FILT_BINS - 1 - threadIdx.x;
+        if (mine < digit) { cnt = 0; sum = 0.0; }
+        else if (mine == digit) { cnt = kept_cnt - above_cnt; sum = kept_sum - above_sum; }
         if (t > floor_key) floor_key = t;                  // (t's open bits are zero: it may lie below the floor it was found above)
         return kept_sum;
     };
@@ -676,9 +735,15 @@ static int sample_filtered_rows(bool all, const float* logits, int ld, int vocab
     if (n_rows <= 0) return 0;
     if (vocab <= 0 || ld < vocab) return VCB_ERR_BAD_ARG;
     if (vocab > (1 << 20)) return VCB_ERR_UNSUPPORTED;      // ids take 20 bits of the key
-    const int ctas = sample_ctas(vocab);
-    return sample_launch(all ? sample_filtered_kernel<true> : sample_filtered_kernel<false>, n_rows, ctas, (cudaStream_t)stream, logits, ld, vocab,
-                         temperature, uniform, top_p, top_k, scratch, out, ctas);
+    // room: a CTA an SM (its registers), less what clusters of four and eight leave unused (us, top-k 50 and top-p 0.9 of 152,064 ids: 8 rows in
+    // eight CTAs 27, in one 62; 64 rows in two 43, in one 64, in eight 111; 256 rows in one 144, in eight 392)
+    const int runs = sample_runs(vocab), lc = sample_ctas_log(vocab, n_rows, 128);
+#define FILTERED(R, ALL) sample_launch(sample_filtered_kernel<R, ALL>, FILT_THREADS, n_rows, lc, (cudaStream_t)stream, logits, ld, vocab, temperature, uniform, top_p, \
+                                       top_k, scratch, out, lc)
+    if (runs == 8) return all ? FILTERED(8, true) : FILTERED(8, false);
+    if (runs == 4) return all ? FILTERED(4, true) : FILTERED(4, false);
+    return all ? FILTERED(1, true) : FILTERED(1, false);
+#undef FILTERED
 }
 
 VCB_EXPORT int vcb_sample_filtered(const float* logits, int ld, int vocab, const float* temperature,
