@@ -86,7 +86,8 @@ def _attention_case(seed, lens, news, nh, nkv, d, page, planes, dtype):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nh,nkv,d,page,planes,window,sink", [
     (2, 2, 4, 16, 2, 0, False), (6, 3, 16, 16, 2, 0, False), (7, 1, 32, 16, 2, 5, False), (18, 2, 36, 32, 2, 0, True), (16, 2, 64, 16, 1, 0, True),
-    (3, 3, 80, 48, 2, 70, False), (28, 4, 128, 16, 2, 0, False), (9, 1, 132, 16, 2, 0, True), (10, 2, 256, 16, 1, 33, False)])
+    (3, 3, 80, 48, 2, 70, False), (28, 4, 128, 16, 2, 0, False), (9, 1, 132, 16, 2, 0, True), (10, 2, 256, 16, 1, 33, False),
+    (12, 4, 84, 16, 2, 0, True), (8, 2, 96, 16, 2, 0, False), (6, 3, 68, 16, 1, 40, True), (5, 5, 96, 16, 2, 0, False), (4, 1, 72, 32, 2, 0, False)])
 def test_attention_rows(ops, dtype, nh, nkv, d, page, planes, window, sink):
     """Groups of one, two and more heads than a warp takes, rows of part of a warp's lanes and of two pieces a lane, keys shared among
     several warps (few tokens) and not (many), windows, sinks, one plane."""
@@ -119,7 +120,7 @@ def test_attention_rows(ops, dtype, nh, nkv, d, page, planes, window, sink):
     ops.check_status()
 
 
-@pytest.mark.parametrize("nh,nkv,d,window", [(4, 4, 32, 0), (14, 2, 128, 0), (8, 1, 256, 90)])
+@pytest.mark.parametrize("nh,nkv,d,window", [(4, 4, 32, 0), (14, 2, 128, 0), (8, 1, 256, 90), (3, 3, 80, 0), (8, 2, 96, 0)])
 def test_attention_rows_do_not_depend_on_the_call(ops, nh, nkv, d, window):
     """A token alone (a warp per part of its keys) and among many (two and four warps, and one, walk the parts) has the same bits, with keys of one
     part, of a few and of eight."""

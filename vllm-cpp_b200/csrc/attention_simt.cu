@@ -437,7 +437,17 @@ static void launch_attention_rows(const AttnArgs& a, cudaStream_t stream) {
 
 template <typename T>
 static void launch_attention_rows(const AttnArgs& a, cudaStream_t stream) {
-    const bool pairs = a.nh / a.nkv <= 2;                  // heads a key's row is read for
+    const int group = a.nh / a.nkv;
+    const bool pairs = group <= 2;                         // heads a key's row is read for
+    if (a.d > 64 && a.d <= 96) {
+        // Rows of 17 to 24 pieces leave a third of the 32 lanes idle: eight lanes hold three pieces each, four keys are read side by side and a
+        // key's product is summed in three exchanges.  One head at a time for one of its own, and in bfloat16 up to three (16 heads of
+        // 80, a prompt of 512, us: with two heads on 32 lanes 566, so 302, the kernel above 445; 24 on 8 638, 409 and 596), four for three and
+        // four (32 on 8 of 96 637, 458 and 1,134); more heads fill eight on 32 lanes (28 on 4 of 80 334, four of them 455), and two in float32
+        // two (407, one 445).
+        if (group == 1 || (sizeof(T) == 2 && group <= 3)) return launch_attention_rows<T, 8, 3, 1>(a, stream);
+        if (group == 3 || group == 4) return launch_attention_rows<T, 8, 3, 4>(a, stream);
+    }
     if (a.d <= 32) pairs ? launch_attention_rows<T, 8, 1, 2>(a, stream) : launch_attention_rows<T, 8, 1, 8>(a, stream);
     else if (a.d <= 64) pairs ? launch_attention_rows<T, 16, 1, 2>(a, stream) : launch_attention_rows<T, 16, 1, 8>(a, stream);
     else if (a.d <= 128) pairs ? launch_attention_rows<T, 32, 1, 2>(a, stream) : launch_attention_rows<T, 32, 1, 8>(a, stream);
