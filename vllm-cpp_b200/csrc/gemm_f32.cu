@@ -343,8 +343,13 @@ VCB_EXPORT int vcb_gemm_f32(const float* A, const float* W, float* C, int M, int
     if (M <= 4) return launch_rows<4, 1, 64, 32>(a, vec, s);
     if (M <= 8 || (long long)M * N * K < (1 << 24)) return launch_rows<8, 1, 64, 32>(a, vec, s);
     if (M <= 16) return N >= 16384 ? launch_rows<16, 1, 128, 32>(a, vec, s) : launch_rows<8, 2, 128, 32>(a, vec, s);
-    // relative time of a tile of 128, 64 and 32 rows: the smaller ones are bound by their shared-memory reads
-    const double t128 = ((M + 127LL) / 128) * 1.0, t64 = ((M + 63LL) / 64) * 0.625, t32 = ((M + 31LL) / 32) * 0.5625;
+    // Relative time of the product in tiles of 128, 64 and 32 rows: where they fill the device, tiles times what one takes of it (the smaller
+    // ones are bound by their shared-memory reads), and at least what one takes alone on its SM: 1,000 rows of [256 x 96] are 16
+    // tiles of 128 rows and 15.7 us, 64 of 32 rows and 8.6; 100 rows of [2,048 x 255] 32.2 and 20.3.  (A tile an SM is where the two meet, taken a
+    // little earlier: 700 rows of [4,096 x 129], 192 tiles of 128 rows 34.9 us, 704 of 32 rows 43.3.)
+    const double wide = (double)((N + 127LL) / 128) * a.slices * 1.4 / vcb_sm_count();
+    const auto time = [&](int rows, double full, double alone) { const double t = full * wide * ((M + rows - 1LL) / rows); return t > alone ? t : alone; };
+    const double t128 = time(128, 1.0, 1.0), t64 = time(64, 0.625, 0.69), t32 = time(32, 0.5625, 0.63);
     if (t128 <= t64 && t128 <= t32) return launch_tiles<8>(a, vec, s);
     return t64 <= t32 ? launch_tiles<4>(a, vec, s) : launch_tiles<2>(a, vec, s);
 }
