@@ -63,7 +63,7 @@ def test_logits_of_infinite_activations(n, width):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n,width,top", [(1, 4, 1), (5, 1028, 3), (7, 1024, 4), (9, 132, 5), (3, 4096, 9), (6, 130, 3)])
+@pytest.mark.parametrize("n,width,top", [(1, 4, 1), (5, 1028, 3), (7, 1024, 4), (9, 132, 5), (3, 4096, 9), (6, 130, 3), (40, 64, 8), (33, 128, 9), (5, 124, 2)])
 def test_combine(n, width, top, dtype):
     from vllm_cpp_b200.csrc import ops
     gen = torch.Generator(device="cuda").manual_seed(n + width)

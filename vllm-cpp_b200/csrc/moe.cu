@@ -967,14 +967,15 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const T* __restr
 }
 
 // The same four elements at a time where the rows allow 4-element pieces: the choices' rows are loaded before the first is used (four at a
-// time), and a token's row is spread over CTAs of 256 pieces.  16 calls of 8 tokens and two of
+// time), and a token's row is spread over CTAs of up to 256 pieces.  Rows below 32 pieces keep the kernel above: its threads of one element have every choice
+// in flight, and half a warp of pieces does not (2,048 tokens, 8 choices, width 64: 3.1 and 5.1 us).  16 calls of 8 tokens and two of
 // 2,048, 4 choices, width 4,096: 347 us one element at a time (each waited for its choice's number and then its row), now 109.
 template <typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_vec_kernel(const float* __restrict__ y, const T* __restrict__ h, long long ldh, const int* __restrict__ pos, const float* __restrict__ wts,
                        T* __restrict__ out, int width, int top, const T* __restrict__ add, long long lda) {
     pdl_start();
-    const int t = blockIdx.x, i = (blockIdx.y * 256 + threadIdx.x) * 4;
+    const int t = blockIdx.x, i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (i >= width) return;
     float4 acc = add ? router_piece<T>(add + (size_t)t * lda + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int k0 = 0; k0 < top; k0 += 4) {
@@ -1006,9 +1007,10 @@ template <typename T>
 static void launch_combine(const float* y, const T* h, long long ldh, const int* pos, const float* wts, T* out, int n_tokens, int width, int top, const T* add,
                            long long lda, cudaStream_t s) {
     const uintptr_t rows = (uintptr_t)h | (uintptr_t)out | (uintptr_t)add;
-    if ((width & 3) == 0 && ((ldh | lda) & 3) == 0 && (((uintptr_t)y) & 15) == 0 && (rows & (4 * sizeof(T) - 1)) == 0 && (width + 1023) / 1024 <= 65535 &&
-        (long long)n_tokens * top <= 0x7fffffffLL) {
-        vcb_launch(moe_combine_vec_kernel<T>, dim3(n_tokens, (width + 1023) / 1024), 256, 0, s, y, h, ldh, pos, wts, out, width, top, add, lda);
+    if (width >= 128 && (width & 3) == 0 && ((ldh | lda) & 3) == 0 && (((uintptr_t)y) & 15) == 0 && (rows & (4 * sizeof(T) - 1)) == 0 &&
+        (width + 1023) / 1024 <= 65535 && (long long)n_tokens * top <= 0x7fffffffLL) {
+        const int threads = width >= 1024 ? 256 : (width / 4 + 31) / 32 * 32;
+        vcb_launch(moe_combine_vec_kernel<T>, dim3(n_tokens, (width / 4 + threads - 1) / threads), threads, 0, s, y, h, ldh, pos, wts, out, width, top, add, lda);
         return;
     }
     vcb_launch(moe_combine_kernel<T>, n_tokens, width >= 1024 ? 256 : 128, 0, s, y, h, ldh, pos, wts, out, width, top, add, lda);
