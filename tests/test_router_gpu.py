@@ -1,4 +1,4 @@
-"""Router logits of few tokens (a warp per output and one or two tokens), of many (two, three and five outputs a warp) and of rows that 4-element pieces do not cover, and the
+"""Router logits of few tokens (a warp per output and one or two tokens), of many (five outputs a warp) and of rows that 4-element pieces do not cover, and the
 choices' rows joined four elements at a time and one at a time; against 64 bits."""
 import pytest
 import torch
@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("n,width,outs", [(1, 4, 3), (8, 1028, 33), (9, 2052, 16), (64, 4096, 40), (65, 4096, 16), (65, 1028, 17), (71, 132, 41), (200, 260, 130),
+@pytest.mark.parametrize("n,width,outs", [(1, 4, 3), (8, 1028, 33), (9, 2052, 16), (64, 4096, 40), (65, 4096, 16), (65, 1028, 17), (71, 132, 41), (200, 260, 130), (700, 516, 33), (160, 516, 130),
                                           (3, 1030, 9), (70, 1030, 9)])
 def test_logits_and_choice(n, width, outs, dtype):
     from vllm_cpp_b200.csrc import ops

@@ -29,8 +29,8 @@
 // kernels with that order, taken by speed alone where 4-element pieces cover the rows:
 //   rows   a warp per output and one or two tokens, eight pieces of both rows in flight a lane: bound by those round trips to L2 (8 tokens, 33
 //          outputs of 4,096: 4.3 us, 12.2 with the last of the three; 128 tokens, 64 outputs: 11.2 and 16.0)
-//   many   eight tokens and two, three or five outputs a warp, so that a token's piece is read for several outputs and a matrix's piece
-//          for eight tokens: bound by the FMAs' operands (2,048 tokens, 33 outputs of 4,096: 35 us, 87 with the kernel below)
+//   many   eight tokens and five outputs a warp, so that a token's piece is read for several outputs and a matrix's piece
+//          for eight tokens: bound by the FMAs' operands (2,048 tokens, 33 outputs of 4,096: 37 us, 87 with the kernel below)
 //   else   a CTA takes RT_TOK tokens and eight router outputs, a warp per output: the tokens' rows pass through shared memory in
 //          slabs (as float); short rows, and those that pieces do not cover.
 // Selection: a warp per token does the softmax over all outputs, adds the correction and
@@ -143,10 +143,10 @@ moe_router_rows_kernel(const T* __restrict__ h, long long ldh, const float* __re
     }
 }
 
-template <typename T, int OUTS>
+template <typename T>
 __global__ void __launch_bounds__(256)
 moe_router_many_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr, float* __restrict__ logits, int n_tokens, int width, int n_out) {
-    constexpr int TOK = 8;
+    constexpr int TOK = 8, OUTS = 5;
     const int t0 = blockIdx.x * TOK, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e0 = (blockIdx.y * 8 + warp) * OUTS;
     pdl_start();
@@ -179,25 +179,20 @@ moe_router_many_kernel(const T* __restrict__ h, long long ldh, const float* __re
 template <typename T>
 static void launch_router_logits(const T* h, long long ldh, const float* wr, float* logits, int n_tokens, int width, int n_out, cudaStream_t s) {
     if ((width & 3) == 0 && (ldh & 3) == 0 && (((uintptr_t)wr) & 15) == 0 && (((uintptr_t)h) & (4 * sizeof(T) - 1)) == 0) {
-        // By the number of logits, measured over 1 to 2,048 tokens, 3 to 256 outputs and widths of 64 to 7,168: a warp each up to 2,500; up to 10,000
-        // a warp for two tokens (64 tokens, 64 outputs of 4,096: 6.6 us, many 18.4), but not for short rows, whose many warps wait for little
-        // each (64 tokens, 130 outputs of 64: 4.0 us, the kernel below 2.7); above, five outputs a warp in float32 (2,048 x 64 of 4,096: 46 us,
-        // three 58), three in bfloat16 (58 and 63 us: its conversions) and where 24 outputs or fewer leave warps of five idle, two for short rows.
+        // By the number of logits, measured over 8 to 2,048 tokens, 8 to 256 outputs and widths of 64 to 7,168 with the matrix out of L2, as a step leaves
+        // it: a warp each up to 2,500; up to 20,000 a warp for two tokens (64 tokens, 64 outputs of 4,096: 10 us, many 32; 256 tokens: 25 and
+        // 31 in float32, 31 and 35 in bfloat16); many above (512 tokens, 64 outputs: 31 and 35 us, a warp for two 41 and 51).  Short rows take the kernel
+        // below instead of a warp for two: many warps would wait for little each (64 tokens, 130 outputs of 64: 2.7 and 4.0 us).
         const long long count = (long long)n_tokens * n_out;
         const auto rows = [&](auto kernel, int tok) {
             const long long items = (long long)((n_tokens + tok - 1) / tok) * n_out;
             vcb_launch(kernel, (unsigned)((items + 7) / 8), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
         };
-        const auto many = [&](auto kernel, int outs) {
-            vcb_launch(kernel, dim3((n_tokens + 7) / 8, (n_out + 8 * outs - 1) / (8 * outs)), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
-        };
         bool taken = true;
         if (count <= 2500) rows(moe_router_rows_kernel<T, 1>, 1);
-        else if (count <= 10000 && width >= 512) rows(moe_router_rows_kernel<T, 2>, 2);
-        else if (count <= 10000) taken = false;
-        else if (width < 512) many(moe_router_many_kernel<T, 2>, 2);
-        else if (sizeof(T) == 4 && count > 20000 && n_out > 24) many(moe_router_many_kernel<T, 5>, 5);
-        else many(moe_router_many_kernel<T, 3>, 3);
+        else if (count > 20000) vcb_launch(moe_router_many_kernel<T>, dim3((n_tokens + 7) / 8, (n_out + 39) / 40), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
+        else if (width >= 512) rows(moe_router_rows_kernel<T, 2>, 2);
+        else taken = false;
         if (taken) return;
     }
     vcb_launch(moe_router_logits_kernel<T>, dim3((n_tokens + RT_TOK - 1) / RT_TOK, (n_out + 7) / 8), 256, 0, s, h, ldh, wr, logits, n_tokens, width, n_out);
