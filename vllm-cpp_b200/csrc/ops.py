@@ -1248,7 +1248,8 @@ def moe_tile_rows(n_tokens: int, top: int, n_experts: int, tensor_cores: bool = 
     None: large), times the pairs at least 4e8.  At that product the two heights cross for every shape measured (8 experts of 1,024, width 2,048, 2
     choices: 64 tokens, 2.7e8, 46.9 against 40.6, 80 tokens, 3.4e8, 46.9 against 49.4; 32 of 256, width 1,024, 4 choices: 256 tokens, 2.7e8, 31.1 against
     30.5, 384, 4.0e8, 31.6 against 33.1; 4 of 512, width 1,024: 800 tokens, 4.2e8, 36.1 against 31.7; 3 of 96, width 64: 22 against 8).  Smaller
-    steps stay at 16 rows: tiles of 64 of so few CTAs are slower (4 of 512, width 1,024, 512 tokens: 42.7 against 29.4)."""
+    steps stay at 16 rows: tiles of 64 of so few CTAs are slower (4 of 512, width 1,024, 512 tokens: 42.7 against 29.4).
+    So 64 rows are for float32 and for bfloat16 whose rows or widths do not fit (one width a multiple of 8 still has its product on ``mma.sync``)."""
     pairs = n_tokens * top
     if tensor_cores and pairs >= 16 * n_experts:
         return 128 if expert_size is None or pairs * expert_size >= 4e8 else 16
@@ -1968,7 +1969,7 @@ def _sample_rows(entry: str, logits, temperature, uniform, top_p, top_k, out, sc
 
 
 def sample_filtered(logits, temperature, uniform, top_p, top_k, out, scratch: Optional[torch.Tensor] = None) -> None:
-    """Redraws, in place in ``out``, the rows that have top-k or top-p set (see sampling.cu).
+    """Redraws, in place in ``out``, the rows that have top-k or top-p set (see sampling.cu); ``sample_all`` is this and ``sample`` in one launch.
     ``scratch``: float32, at least rows * vocab elements; one is kept and grown here if not given."""
     _sample_rows("vcb_sample_filtered", logits, temperature, uniform, top_p, top_k, out, scratch)
 

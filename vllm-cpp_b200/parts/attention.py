@@ -47,8 +47,8 @@ class PagedAttentionKernels(Mixer):
         if self.dtype == torch.bfloat16 and self.d not in ops.MMA_HEAD_DIMS and self.d not in _warned_head_dims:
             _warned_head_dims.add(self.d)
             print(f"[vllm_cpp_b200] warning: head size {self.d} has no tensor-core attention kernel "
-                  f"(those take {ops.MMA_HEAD_DIMS}); bfloat16 attention runs the plain kernel, one warp per "
-                  "token and head, many times slower", file=sys.stderr, flush=True)
+                  f"(those take {ops.MMA_HEAD_DIMS}); bfloat16 attention runs the plain kernel on the FMA "
+                  "pipe, many times slower for prompts", file=sys.stderr, flush=True)
 
     def step_arrays(self):
         """What the kernels need per step beyond the common arrays, built on the host from the step's
