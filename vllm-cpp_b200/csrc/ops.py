@@ -1245,9 +1245,11 @@ def moe_tile_rows(n_tokens: int, top: int, n_experts: int, tensor_cores: bool = 
     moe_tensor_tiles finds fit): 128 rows, the tcgen05 products, from 16 tokens an expert on (both products, us: 32 experts of 2,048,
     width 4,096, 4 choices, 128 tokens 274 against 344 with 16 rows, 512 tokens 292 against 656 with 64), if the step's products are large
     enough for a CTA of 128 x 256 sums to be worth its start: ``expert_size``, the elements of an expert's matrix (width times size;
-    None: large), times the pairs at least 4e8.  At that product the two heights cross for every shape measured (8 experts of 1,024, width 2,048, 2
+    None: large), times the pairs at least 4e8.  Around that product the two heights cross (8 experts of 1,024, width 2,048, 2
     choices: 64 tokens, 2.7e8, 46.9 against 40.6, 80 tokens, 3.4e8, 46.9 against 49.4; 32 of 256, width 1,024, 4 choices: 256 tokens, 2.7e8, 31.1 against
-    30.5, 384, 4.0e8, 31.6 against 33.1; 4 of 512, width 1,024: 800 tokens, 4.2e8, 36.1 against 31.7; 3 of 96, width 64: 22 against 8).  Smaller
+    30.5, 384, 4.0e8, 31.6 against 33.1; 4 of 512, width 1,024: 800 tokens, 4.2e8, 36.1 against 31.7; 3 of 96, width 64: 22 against 8).  Of 67
+    sizes of ten shapes, 64 to 4,096 tokens, the rule took the best height for 64; the others are narrow experts of many pairs below the line (64 of 128, width
+    512, 8 choices, 512 tokens, 2.7e8: 28.9 where 128 rows take 24.4; 8 of 128, width 256, 4,096 tokens: 28.2 and 24.3; 8 of 256, width 128: 30.8 and, with 64, 28.5).  Smaller
     steps stay at 16 rows: tiles of 64 of so few CTAs are slower (4 of 512, width 1,024, 512 tokens: 42.7 against 29.4).
     So 64 rows are for float32 and for bfloat16 whose rows or widths do not fit (one width a multiple of 8 still has its product on ``mma.sync``)."""
     pairs = n_tokens * top
